@@ -26,6 +26,12 @@ inline unsigned __float_as_uint(float f) { unsigned u; std::memcpy(&u, &f, 4); r
 inline int __float_as_int(float f) { int u; std::memcpy(&u, &f, 4); return u; }
 inline float __uint_as_float(unsigned u) { float f; std::memcpy(&f, &u, 4); return f; }
 inline float __int_as_float(int u) { float f; std::memcpy(&f, &u, 4); return f; }
+inline unsigned __byte_perm(unsigned a, unsigned b, unsigned sel) {
+    const unsigned long long v = (static_cast<unsigned long long>(b) << 32) | a;
+    unsigned r = 0;
+    for (int i = 0; i < 4; ++i) r |= static_cast<unsigned>((v >> (8 * ((sel >> (4 * i)) & 7u))) & 255u) << (8 * i);
+    return r;
+}
 inline void sincospif(float x, float* s, float* c) {
     const double a = 3.14159265358979323846 * double(x);
     *s = float(std::sin(a));

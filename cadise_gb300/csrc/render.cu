@@ -16,6 +16,7 @@
 #include "film.cuh"
 #include "internal.h"
 #include "pathtrace.cuh"
+#include "persist.cuh"
 #include "radix.cuh"
 
 #include <algorithm>
@@ -396,125 +397,55 @@ __global__ void k_wf_extend_dyn(RenderArgs a, int b) {
     count_flush<COUNT>(a.counters, tc, TraceCounters{0, 0}, nclosest, 0);
 }
 
-// Persistent closest-hit pass: the while-while traversal of traverse_warp
-// with dynamic ray fetch (Aila & Laine 2009).  A lane keeps its ray across
-// rounds; after each round of leaves, once fewer than a.refill_closest lanes
-// of the warp still hold an unfinished ray (the autotuned compaction
-// threshold), the finished lanes store their hits and take the next rays of
-// the queue, so lanes do not idle until the warp's longest ray is done.
-// Same hits as the other extend kernels (closer_hit).
+// Registers of the persistent passes: 18 blocks of 64 threads an SM.  The
+// 1 M-triangle frame's closest-hit passes take 33.9 ms at 56 registers (20 bytes
+// of spills in the ray set-up), 34.6 at 64 and 37.3 at 48.
+constexpr int kPersistRegs = 56;
 
-// At most 56 registers a thread (a few spilled values, in the ray set-up):
-// 18 blocks of 64 threads fit an SM instead of 12, and the closest-hit pass
-// then runs beside the any-hit pass with more warps to hide its L1 / L2
-// latency (samples/s on the 1 M-triangle frame: +4.5 % at 64 registers,
-// +7.0 % at 56, against the uncapped 75).
+// Persistent closest-hit pass (persist.cuh) over the continuation rays.  A ray
+// that meets two primitives within the tie window is left to k_wf_ties.
 template <bool COUNT, bool SPH, bool SORTED = false, bool ADJ = false>
-__global__ void __maxnreg__(56) k_wf_extend_pww(RenderArgs a, int b) {
+__global__ void __maxnreg__(kPersistRegs) k_wf_extend_pww(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
     int* cnt = w.cnt + b * kCntStride;
-    const int ncont = cnt[0], nmis = cnt[1];
-    const int n = ncont + nmis;
+    const int n = cnt[0];
     const int* qc = w.q_cont[b & 1];
-    const int* qm = w.q_mis[b & 1];
-    int* const* qmat = w.q_mat;
     TraceCounters tc{0, 0};
     uint32_t nclosest = 0;
-    SharedStack<true> stack;
-    stack.bind();
-    int sp = 0;
-    RayPre r{};
-    float tcur = 0.0f, hu = 0.0f, hv = 0.0f;
-    int hslot = -1;
-    uint32_t cur = kNoEntry, leaf = kNoEntry;
-    int i = -1, p = -1;  // queue entry and path of this lane's ray (i < 0: none)
-    bool cont = false;   // continuation ray (else MIS ray)
-    bool drained = false;
-    uint32_t left = 0;  // node and leaf visits this ray has left (over_budget)
-    auto pop = [&]() -> uint32_t {
-        while (sp > 0) {
-            --sp;
-            if (stack.dist(sp) <= tcur * 1.00000036f) return stack.entry(sp);
-        }
-        return kNoEntry;
-    };
-    for (;;) {
-        const bool need = i < 0 && !drained;
-        const int k = warp_take(cnt + 8, need, n);
-        if (need) {
-            if (k < 0) {
-                drained = true;
-            } else {
-                i = k;
-                p = extend_entry<SORTED>(a, qc, qm, ncont, i, &cont);
-                const float3 o = f3(__ldcs(&w.ray_o[p]));
-                const float3 d = cont ? f3(__ldcs(&w.ray_d[p])) : f3(__ldcs(&w.mis_d[p]));
-                r = ray_prep(o, d, kRayEps, kFloatMax);
-                tcur = r.tmax;
-                hslot = -1;
-                hu = hv = 0.0f;
-                cur = 0;
-                leaf = kNoEntry;
-                sp = 0;
-                left = a.scenes[__ldcs(&w.meta[p].x)].visit_budget;
-                if (COUNT) ++nclosest;
-            }
-        }
-        if (__all_sync(__activemask(), i < 0)) break;
-        if (i < 0) continue;
-        const SceneD& S = a.scenes[__ldcs(&w.meta[p].x)];
-        for (;;) {
-            while (cur != kNoEntry && !entry_is_leaf(cur)) {
-                if (over_budget(S, left)) {
-                    cur = leaf = kNoEntry;
-                    break;
-                }
-                cur = visit_node<false, COUNT, false>(S, r, cur, tcur, stack, sp, &tc);
-                if (cur == kNoEntry) cur = pop();
-                if (leaf == kNoEntry && cur != kNoEntry && entry_is_leaf(cur)) {
-                    leaf = cur;
-                    cur = pop();
-                }
-                if (!__any_sync(__activemask(), leaf == kNoEntry)) break;
-            }
-            if (leaf == kNoEntry) {
-                if (cur == kNoEntry) break;  // the ray is done
-                leaf = cur;
-                cur = pop();
-            }
-            while (leaf != kNoEntry) {
-                if (over_budget(S, left)) {
-                    cur = leaf = kNoEntry;
-                    break;
-                }
-                visit_leaf<false, COUNT, SPH, true>(S, r, leaf, tcur, hslot, hu, hv, &tc);
-                leaf = kNoEntry;
-                if (cur != kNoEntry && entry_is_leaf(cur)) {
-                    leaf = cur;
-                    cur = pop();
-                }
-            }
-            if (cur == kNoEntry) break;  // the ray is done
-            if (__popc(__activemask()) < a.refill_closest) break;
-        }
-        if (cur == kNoEntry && leaf == kNoEntry) {
-            if (hu != 0.0f) {
-                // two primitives within the tie window: k_wf_ties decides
-                w.q_tie[atomicAdd(cnt + 12, 1)] = cont ? p : int(uint32_t(p) | 0x80000000u);
+    persistent_pass<false, COUNT, SPH>(
+        a.scenes, cnt + 8, n, a.refill_closest, kRayEps,
+        [&](int k, float3* o, float3* d, float* tmax, int* scene) {
+            bool cont;
+            const int p = extend_entry<SORTED>(a, qc, nullptr, n, k, &cont);
+            *o = f3(__ldcs(&w.ray_o[p]));
+            *d = f3(__ldcs(&w.ray_d[p]));
+            *scene = int(__ldcs(&w.meta[p].x));
+            *tmax = kFloatMax;
+            if (COUNT) ++nclosest;
+            return p;
+        },
+        [&](bool done, int p, float t, int slot, bool tie) {
+            if (!done) return;
+            if (tie) {
+                w.q_tie[atomicAdd(cnt + 12, 1)] = p;
             } else {
                 HitD hit;
-                hit.t = tcur;
-                hit.slot = hslot;
-                // the shading recomputes the surface coordinates from the hit
-                // point (hit_point), so the traversal's need not be kept
+                hit.t = t;
+                hit.slot = slot;
                 hit.u = 0.0f;
                 hit.v = 0.0f;
-                const int key = extend_finish<ADJ>(w, S, p, cont, r.o, r.d, hslot >= 0, hit, &a.adj);
-                grouped_push(qmat, cnt + 3, key, p);
+                const SceneD& S = a.scenes[__ldcs(&w.meta[p].x)];
+                const float3 o = splat3(0.0f);
+                const float3 d = S.env_light >= 0 ? f3(__ldcs(&w.ray_d[p])) : splat3(0.0f);
+                const int key = extend_finish<ADJ>(w, S, p, true, o, d, slot >= 0, hit, &a.adj);
+                grouped_push(w.q_mat, cnt + 3, key, p);
             }
-            i = -1;
-        }
-    }
+        },
+        [&](int p) {
+            uint32_t* st = a.scenes[w.meta[p].x].status;
+            if (st) atomicAdd(st, 1u);
+        },
+        tc);
     count_flush<COUNT>(a.counters, tc, TraceCounters{0, 0}, nclosest, 0);
 }
 
@@ -554,99 +485,36 @@ __global__ void k_wf_ties(RenderArgs a, int b) {
     if (COUNT && nties) atomicAdd(a.counters + 6, (unsigned long long)nties);
 }
 
-// Persistent any-hit pass: k_wf_extend_pww's while-while traversal with
-// dynamic ray fetch for the shadow rays; a ray ends at its first hit.  The
-// refill threshold is a.refill_any.
+// Persistent any-hit pass over the shadow rays; a ray ends at its first hit.
 
 template <bool COUNT, bool SPH, bool ADJ = false>
-__global__ void k_wf_shadow_pww(RenderArgs a, int b) {
+__global__ void __maxnreg__(kPersistRegs) k_wf_shadow_pww(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
     int* cnt = w.cnt + b * kCntStride;
     const int n = cnt[2];
     const int* q = w.q_shadow[b & 1];
     TraceCounters tc{0, 0};
     uint32_t nany = 0;
-    SharedStack<false> stack;
-    stack.bind();
-    int sp = 0;
-    RayPre r{};
-    float tcur = 0.0f, hu = 0.0f, hv = 0.0f;
-    int hslot = -1;
-    uint32_t cur = kNoEntry, leaf = kNoEntry;
-    int i = -1, p = -1;
-    bool occluded = false, drained = false;
-    uint32_t left = 0;  // node and leaf visits this ray has left (over_budget)
-    auto pop = [&]() -> uint32_t {
-        if (sp > 0) return stack.entry(--sp);
-        return kNoEntry;
-    };
-    for (;;) {
-        const bool need = i < 0 && !drained;
-        const int k = warp_take(cnt + 9, need, n);
-        if (need) {
-            if (k < 0) {
-                drained = true;
-            } else {
-                i = k;
-                p = q[i];
-                const float4 sd = __ldcs(&w.sh_d[p]);
-                r = ray_prep(f3(__ldcs(&w.ray_o[p])), f3(sd), kRayEps, sd.w);
-                tcur = r.tmax;
-                hslot = -1;
-                cur = 0;
-                leaf = kNoEntry;
-                sp = 0;
-                occluded = false;
-                left = a.scenes[__ldcs(&w.meta[p].x)].visit_budget;
-                if (COUNT) ++nany;
-            }
-        }
-        if (__all_sync(__activemask(), i < 0)) break;
-        if (i < 0) continue;
-        const SceneD& S = a.scenes[__ldcs(&w.meta[p].x)];
-        for (;;) {
-            while (cur != kNoEntry && !entry_is_leaf(cur)) {
-                if (over_budget(S, left)) {
-                    cur = leaf = kNoEntry;
-                    break;
-                }
-                cur = visit_node<true, COUNT>(S, r, cur, tcur, stack, sp, &tc);
-                if (cur == kNoEntry) cur = pop();
-                if (leaf == kNoEntry && cur != kNoEntry && entry_is_leaf(cur)) {
-                    leaf = cur;
-                    cur = pop();
-                }
-                if (!__any_sync(__activemask(), leaf == kNoEntry)) break;
-            }
-            if (leaf == kNoEntry) {
-                if (cur == kNoEntry) break;  // the ray is done: unoccluded
-                leaf = cur;
-                cur = pop();
-            }
-            while (leaf != kNoEntry) {
-                if (over_budget(S, left)) {
-                    cur = leaf = kNoEntry;
-                    break;
-                }
-                if (visit_leaf<true, COUNT, SPH>(S, r, leaf, tcur, hslot, hu, hv, &tc)) {
-                    occluded = true;
-                    cur = leaf = kNoEntry;
-                    break;
-                }
-                leaf = kNoEntry;
-                if (cur != kNoEntry && entry_is_leaf(cur)) {
-                    leaf = cur;
-                    cur = pop();
-                }
-            }
-            if (cur == kNoEntry) break;  // the ray is done
-            if (__popc(__activemask()) < a.refill_any) break;
-        }
-        if (cur == kNoEntry && leaf == kNoEntry) {
-            shadow_finish<ADJ>(w, p, occluded);
-            i = -1;
-        }
-    }
+    persistent_pass<true, COUNT, SPH>(
+        a.scenes, cnt + 9, n, a.refill_any, kRayEps,
+        [&](int k, float3* o, float3* d, float* tmax, int* scene) {
+            const int p = q[k];
+            const float4 sd = __ldcs(&w.sh_d[p]);
+            *o = f3(__ldcs(&w.ray_o[p]));
+            *d = f3(sd);
+            *tmax = sd.w;
+            *scene = int(__ldcs(&w.meta[p].x));
+            if (COUNT) ++nany;
+            return p;
+        },
+        [&](bool done, int p, float, int slot, bool) {
+            if (done) shadow_finish<ADJ>(w, p, slot >= 0);
+        },
+        [&](int p) {
+            uint32_t* st = a.scenes[w.meta[p].x].status;
+            if (st) atomicAdd(st, 1u);
+        },
+        tc);
     count_flush<COUNT>(a.counters, TraceCounters{0, 0}, tc, 0, nany);
 }
 
@@ -1044,7 +912,7 @@ int grid_for(cgpu_ctx* ctx, K kernel, int block, uint64_t work, size_t shared_by
 template <typename K>
 size_t stack_smem(K kernel, bool shared_stack, bool with_t, int block) {
     if (!shared_stack) return 0;
-    const size_t bytes = with_t ? SharedStack<true>::bytes(block) : SharedStack<false>::bytes(block);
+    const size_t bytes = with_t ? persist_bytes(block, true) : persist_bytes(block, false);
     if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
     return bytes;
 }

@@ -24,7 +24,8 @@ struct __align__(16) Bvh4Node {
     uint32_t exps;      // bytes 0..2: biased exponents e of the x, y, z steps 2^(e - 127)
     uint32_t child[4];
     uint32_t lox, hix, loy, hiy;  // byte i: child i's plane in steps from the origin
-    uint32_t loz, hiz, pad0, pad1;
+    uint32_t loz, hiz;
+    float stepy, stepz;  // the y and z steps again, as floats
 };
 static_assert(sizeof(Bvh4Node) == 64, "Bvh4Node is 64 bytes");
 
@@ -84,7 +85,8 @@ CG_HD void quantize_node(const float (&lo)[4][3], const float (&hi)[4][3], const
     out->hiy = qhi[1];
     out->loz = qlo[2];
     out->hiz = qhi[2];
-    out->pad0 = out->pad1 = 0u;
+    out->stepy = float(ldexp(1.0, int(ebits[1]) - 127));
+    out->stepz = float(ldexp(1.0, int(ebits[2]) - 127));
 }
 
 constexpr uint32_t kLeafBit = 0x80000000u;

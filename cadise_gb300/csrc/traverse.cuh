@@ -88,6 +88,39 @@ CG_D bool tri_test(const RayPre& r, float3 A3, float3 B3, float3 C3, float tcur,
     return true;
 }
 
+// tri_test with the axes rotated, not permuted, so that kz is the last: where
+// tri_test swaps kx and ky (d[kz] < 0) every edge function, the determinant and
+// T change sign exactly, and its own sign change of a negative determinant
+// undoes that, so t and the decision are tri_test's to the bit.
+CG_D bool tri_test_rot(float3 o, int kz, float Sx, float Sy, float Sz, float tmin, float3 A3, float3 B3, float3 C3,
+                       float tcur, float* tout) {
+    const float3 A = A3 - o, B = B3 - o, C = C3 - o;
+    const bool k0 = kz == 0, k1 = kz == 1;
+    const float Akz = k0 ? A.x : k1 ? A.y : A.z, Bkz = k0 ? B.x : k1 ? B.y : B.z, Ckz = k0 ? C.x : k1 ? C.y : C.z;
+    const float Ax = (k0 ? A.y : k1 ? A.z : A.x) - Sx * Akz;
+    const float Ay = (k0 ? A.z : k1 ? A.x : A.y) - Sy * Akz;
+    const float Bx = (k0 ? B.y : k1 ? B.z : B.x) - Sx * Bkz;
+    const float By = (k0 ? B.z : k1 ? B.x : B.y) - Sy * Bkz;
+    const float Cx = (k0 ? C.y : k1 ? C.z : C.x) - Sx * Ckz;
+    const float Cy = (k0 ? C.z : k1 ? C.x : C.y) - Sy * Ckz;
+    float U = __fsub_rn(__fmul_rn(Cx, By), __fmul_rn(Cy, Bx));
+    float V = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
+    float W = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
+    if (U == 0.0f || V == 0.0f || W == 0.0f) {
+        U = float(double(Cx) * double(By) - double(Cy) * double(Bx));
+        V = float(double(Ax) * double(Cy) - double(Ay) * double(Cx));
+        W = float(double(Bx) * double(Ay) - double(By) * double(Ax));
+    }
+    const float det = U + V + W;
+    float T = U * (Sz * Akz) + V * (Sz * Bkz) + W * (Sz * Ckz);
+    if (det < 0.0f) T = -T;
+    const float ad = fabsf(det);
+    const bool mixed = fminf(fminf(U, V), W) < 0.0f && fmaxf(fmaxf(U, V), W) > 0.0f;
+    if (mixed || ad == 0.0f || T < tmin * ad || T > tcur * ad) return false;
+    *tout = T * (1.0f / ad);
+    return true;
+}
+
 struct HitD {
     float t;
     int slot;  // triangle slot in leaf order, -1 on a miss
@@ -104,12 +137,23 @@ CG_D float4 ldg4(const float4* p) { return __ldg(p); }
 // Loads node `idx`: q[0] the frame origin and step exponents, q[1] the four
 // child entries, q[2] / q[3] the quantized planes (lo / hi x, lo / hi y,
 // lo / hi z).
-CG_D void load_node(const Bvh4Node* nodes, uint32_t idx, const RayPre& r, float4 (&q)[4]) {
+CG_D void load_node(const Bvh4Node* nodes, uint32_t idx, float4 (&q)[4]) {
     const float4* p = reinterpret_cast<const float4*>(nodes + idx);
+#if defined(__CUDA_ARCH__)
+    // two 32-byte loads: half the L1 requests of four 16-byte ones (closest-hit
+    // passes of the 1 M-triangle frame 40.9 -> 39.7 ms)
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(q[0].x), "=f"(q[0].y), "=f"(q[0].z), "=f"(q[0].w), "=f"(q[1].x), "=f"(q[1].y), "=f"(q[1].z), "=f"(q[1].w)
+        : "l"(p));
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(q[2].x), "=f"(q[2].y), "=f"(q[2].z), "=f"(q[2].w), "=f"(q[3].x), "=f"(q[3].y), "=f"(q[3].z), "=f"(q[3].w)
+        : "l"(p + 2));
+#else
     q[0] = __ldg(p + 0);
     q[1] = __ldg(p + 1);
     q[2] = __ldg(p + 2);
     q[3] = __ldg(p + 3);
+#endif
 }
 
 // Closest-hit tie window (tie_prefers): candidates whose distances lie within
@@ -122,39 +166,43 @@ CG_D void load_node(const Bvh4Node* nodes, uint32_t idx, const RayPre& r, float4
 constexpr float kTieSlack = 1.000004f;
 CG_D float tie_hi(const SceneD& S, float t) { return t * kTieSlack + S.tie_abs; }
 
+// Box tests widen by 1 + 10 x 2^-24: three roundings of each plane's distance,
+// and one more each for a reciprocal unit's 1 / d.
+constexpr float kBoxSlack = 1.0000006f;
+
 // Child box distances; tnear = +inf marks a miss.  Empty child slots hold
 // entry 0 (the root, never anyone's child) and are always a miss.  Per axis
 // the slab distances are a + q * b with a = (origin - o) / d and b = step / d
 // (exact: the step is a power of two), the near plane picked by the sign of d.
-CG_D void child_hits(const RayPre& r, const float4 (&q)[4], float tcur, float (&tn)[4]) {
+CG_D void child_hits(float3 o, float3 inv, float tmin, const float4 (&q)[4], float tcur, float (&tn)[4]) {
     const uint32_t ce[4] = {__float_as_uint(q[1].x), __float_as_uint(q[1].y), __float_as_uint(q[1].z),
                             __float_as_uint(q[1].w)};
     const uint32_t exps = __float_as_uint(q[0].w);
-    const float bx = __uint_as_float((exps & 255u) << 23) * r.inv.x;
-    const float by = __uint_as_float(((exps >> 8) & 255u) << 23) * r.inv.y;
-    const float bz = __uint_as_float(((exps >> 16) & 255u) << 23) * r.inv.z;
-    const float ax = (q[0].x - r.o.x) * r.inv.x;
-    const float ay = (q[0].y - r.o.y) * r.inv.y;
-    const float az = (q[0].z - r.o.z) * r.inv.z;
+    const float bx = fabsf(__uint_as_float(exps << 23)) * inv.x;
+    const float by = q[3].z * inv.y, bz = q[3].w * inv.z;
+    const float ax = (q[0].x - o.x) * inv.x;
+    const float ay = (q[0].y - o.y) * inv.y;
+    const float az = (q[0].z - o.z) * inv.z;
     // 1 where the ray runs towards -axis: the near plane is the upper one
-    const bool sx = (__float_as_uint(r.inv.x) >> 31) != 0u, sy = (__float_as_uint(r.inv.y) >> 31) != 0u,
-               sz = (__float_as_uint(r.inv.z) >> 31) != 0u;
+    const bool sx = (__float_as_uint(inv.x) >> 31) != 0u, sy = (__float_as_uint(inv.y) >> 31) != 0u,
+               sz = (__float_as_uint(inv.z) >> 31) != 0u;
     const uint32_t lox = __float_as_uint(q[2].x), hix = __float_as_uint(q[2].y);
     const uint32_t loy = __float_as_uint(q[2].z), hiy = __float_as_uint(q[2].w);
     const uint32_t loz = __float_as_uint(q[3].x), hiz = __float_as_uint(q[3].y);
     const uint32_t nx = sx ? hix : lox, fx = sx ? lox : hix;
     const uint32_t ny = sy ? hiy : loy, fy = sy ? loy : hiy;
     const uint32_t nz = sz ? hiz : loz, fz = sz ? loz : hiz;
-    const float tlim = tcur * 1.00000036f;  // 1 + 2 gamma(3)
+    const float tlim = tcur * kBoxSlack;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int sh = 8 * i;
         const float tnx = fmaf(float((nx >> sh) & 255u), bx, ax), tfx = fmaf(float((fx >> sh) & 255u), bx, ax);
         const float tny = fmaf(float((ny >> sh) & 255u), by, ay), tfy = fmaf(float((fy >> sh) & 255u), by, ay);
         const float tnz = fmaf(float((nz >> sh) & 255u), bz, az), tfz = fmaf(float((fz >> sh) & 255u), bz, az);
-        const float tnear = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, r.tmin));
+        const float tnear = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, tmin));
         const float tfar = fminf(fminf(tfx, tfy), fminf(tfz, tlim));
-        tn[i] = (ce[i] != 0u && tnear <= tfar * 1.00000036f) ? tnear : __int_as_float(0x7f800000);
+        // slot 0 is never empty
+        tn[i] = ((i == 0 || ce[i] != 0u) && tnear <= tfar * kBoxSlack) ? tnear : __int_as_float(0x7f800000);
     }
 }
 
@@ -179,7 +227,8 @@ CG_D bool over_budget(const SceneD& S, uint32_t& left) {
 // Traversal stacks: kStackSize entries of (child entry, entry distance),
 // enough for any tree the upload accepts (3 x depth + 1 entries).
 // LocalStack keeps them in per-thread arrays (local memory on the GPU): the
-// megakernel, the per-ray loops and the host build of these headers.
+// megakernel, the per-ray loops and the host build of these headers (the
+// persistent passes have their own, persist.cuh).
 struct LocalStack {
     uint32_t e[kStackSize];
     float t[kStackSize];
@@ -188,63 +237,17 @@ struct LocalStack {
     CG_HD float dist(int sp) const { return t[sp]; }
 };
 
-#ifdef __CUDACC__
-// The persistent traversal passes keep the bottom kSmemStack entries of each
-// lane in shared memory and only deeper ones in local memory: on the 1 M-
-// triangle field a closest-hit ray's stack reaches 4 entries at the median,
-// 10 at the 99th percentile and more than 16 for 2 rays in 100,000.  Each
-// warp owns kSmemStack rows of 32 words (64 with distances: the 32 entries,
-// then their 32 distances); entry k of lane l sits at word
-// row_base + k * row + l, so the lanes of a warp always hit 32 different
-// banks whatever depth each one is at, and one register (the lane's base)
-// addresses the whole stack.  WITH_T = false (any-hit) keeps no distances:
-// an any-hit pass pops without the distance test.
-constexpr int kSmemStack = 16;
-// the dynamic shared memory of a persistent traversal launch
-extern __shared__ uint32_t trav_stack_smem[];
-
-template <bool WITH_T>
-struct SharedStack {
-    static constexpr int kRow = WITH_T ? 64 : 32;  // words per stack level of a warp
-    uint32_t base;   // this lane's word of level 0
-    uint32_t oe[kStackSize - kSmemStack];
-    float ot[WITH_T ? kStackSize - kSmemStack : 1];
-
-    // Shared memory per block for `threads` threads (a multiple of 32).
-    static constexpr size_t bytes(int threads) { return size_t(threads) * kSmemStack * (WITH_T ? 8u : 4u); }
-    CG_D void bind() { base = (threadIdx.x >> 5) * uint32_t(kSmemStack * kRow) + (threadIdx.x & 31u); }
-    CG_D void push(int sp, uint32_t ee, float tt) {
-        if (sp < kSmemStack) {
-            trav_stack_smem[base + sp * kRow] = ee;
-            if (WITH_T) trav_stack_smem[base + sp * kRow + 32] = __float_as_uint(tt);
-        } else {
-            oe[sp - kSmemStack] = ee;
-            if (WITH_T) ot[sp - kSmemStack] = tt;
-        }
-    }
-    CG_D uint32_t entry(int sp) const {
-        return sp < kSmemStack ? trav_stack_smem[base + sp * kRow] : oe[sp - kSmemStack];
-    }
-    CG_D float dist(int sp) const {
-        if (!WITH_T) return 0.0f;
-        return sp < kSmemStack ? __uint_as_float(trav_stack_smem[base + sp * kRow + 32]) : ot[sp - kSmemStack];
-    }
-};
-#endif
-
 // Visits inner node `e`: pushes the children the ray enters, farthest first,
 // except the nearest, which it returns (kNoEntry when the ray misses all four).
-// WIDE = false (the persistent closest-hit pass, which leaves ties to
-// k_wf_ties): children culled by tcur itself, not by the tie window.
-template <bool ANY, bool COUNT, bool WIDE = true, typename Stack>
+template <bool ANY, bool COUNT, typename Stack>
 CG_D uint32_t visit_node(const SceneD& S, const RayPre& r, uint32_t e, float tcur, Stack& stack, int& sp,
                          TraceCounters* cnt) {
     const float kInf = __int_as_float(0x7f800000);
     float4 q[4];
-    load_node(S.nodes, e, r, q);
+    load_node(S.nodes, e, q);
     if (COUNT) cnt->nodes++;
     float tn[4];
-    child_hits(r, q, (ANY || !WIDE) ? tcur : tie_hi(S, tcur), tn);
+    child_hits(r.o, r.inv, r.tmin, q, ANY ? tcur : tie_hi(S, tcur), tn);
     uint32_t ce[4] = {__float_as_uint(q[1].x), __float_as_uint(q[1].y), __float_as_uint(q[1].z),
                       __float_as_uint(q[1].w)};
     if (!ANY) {
@@ -400,12 +403,7 @@ CG_D bool closer_hit(const SceneD& S, const RayPre& r, float t, int prim, int sl
 // SPH = false: the scene holds no spheres, and the sphere test is compiled out
 // of the hot kernels (a sphere record would then be misread as a triangle, so
 // the host picks SPH from the scenes it renders).
-// DEFER (the persistent closest-hit pass): the watertight rule alone, and hu
-// set to 1 when a candidate lies within the tie window of the kept hit - the
-// ray is then traced again by k_wf_ties with tie_prefers - so that the rare
-// tie code stays out of that register-capped kernel.  hu / hv are not the
-// hit's coordinates there.
-template <bool ANY, bool COUNT, bool SPH = true, bool DEFER = false>
+template <bool ANY, bool COUNT, bool SPH = true>
 CG_D bool visit_leaf(const SceneD& S, const RayPre& r, uint32_t e, float& tcur, int& hslot, float& hu, float& hv,
                      TraceCounters* cnt) {
     const uint32_t first = leaf_first(e), n = leaf_count(e);
@@ -425,13 +423,7 @@ CG_D bool visit_leaf(const SceneD& S, const RayPre& r, uint32_t e, float& tcur, 
                 tcur = t;
                 return true;
             }
-            if (DEFER) {
-                if (hslot >= 0 && tie_hi(S, t) >= tcur) hu = 1.0f;
-                if (hslot < 0 ? t <= tcur : (t < tcur || (t == tcur && slot < hslot))) {
-                    hslot = slot;
-                    tcur = t;
-                }
-            } else if (closer_hit(S, r, t, __float_as_int(a.w), slot, tcur, hslot)) {
+            if (closer_hit(S, r, t, __float_as_int(a.w), slot, tcur, hslot)) {
                 hslot = slot;
                 tcur = t;
                 hu = u;
@@ -470,7 +462,7 @@ CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* c
         // else the next stack entry that can still hold a closer hit
         while (next == kNoEntry && sp > 0) {
             --sp;
-            if (ANY || stack.dist(sp) <= tie_hi(S, tcur) * 1.00000036f) next = stack.entry(sp);
+            if (ANY || stack.dist(sp) <= tie_hi(S, tcur) * kBoxSlack) next = stack.entry(sp);
         }
         if (next == kNoEntry) break;
         cur = next;
@@ -557,7 +549,7 @@ CG_D bool traverse_warp(const SceneD& S, const RayPre& r, HitD* hit, TraceCounte
     auto pop = [&]() -> uint32_t {
         while (sp > 0) {
             --sp;
-            if (stack.dist(sp) <= tie_hi(S, tcur) * 1.00000036f) return stack.entry(sp);
+            if (stack.dist(sp) <= tie_hi(S, tcur) * kBoxSlack) return stack.entry(sp);
         }
         return kNoEntry;
     };
@@ -647,7 +639,7 @@ CG_D void trav_step(const SceneD& S, const RayPre& r, TravState& st, TraceCounte
     }
     while (st.sp > 0) {
         --st.sp;
-        if (ANY || st.stack.dist(st.sp) <= tie_hi(S, st.tcur) * 1.00000036f) {
+        if (ANY || st.stack.dist(st.sp) <= tie_hi(S, st.tcur) * kBoxSlack) {
             st.cur = st.stack.entry(st.sp);
             return;
         }
