@@ -124,6 +124,7 @@ cgpu_status cgpu_params_get(cgpu_ctx* ctx, int32_t scene, float* texels, float* 
         size_t off = 0;
         for (const TextureD& t : sl.h_texs) {
             const size_t n = size_t(t.width) * t.height * 3;
+            cg_prefault(texels + off, n * sizeof(float));
             cudaError_t e = cudaMemcpy(texels + off, t.texels, n * sizeof(float), cudaMemcpyDeviceToHost);
             if (e != cudaSuccess) return cg_cuda(ctx, e, "params_get texels");
             off += n;
@@ -295,6 +296,7 @@ cgpu_status cgpu_adjoint_backward(cgpu_ctx* ctx, int32_t scene, uint32_t spp, ui
         e = cudaGetLastError();
         ctx->stats.kernel_launches = 1;
     }
+    if (e == cudaSuccess && grad_texels && ntex) cg_prefault(grad_texels, ntex * sizeof(double));
     if (e == cudaSuccess && grad_texels && ntex)
         e = cudaMemcpyAsync(grad_texels, d_gt, ntex * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess && grad_roughness)

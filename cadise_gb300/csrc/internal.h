@@ -300,6 +300,7 @@ void cg_free_render_state(cgpu_ctx* ctx);
 cgpu_status cg_fail(cgpu_ctx* ctx, cgpu_status s, const std::string& msg);
 cgpu_status cg_cuda(cgpu_ctx* ctx, cudaError_t e, const char* what);
 cgpu_status cg_sync_tables(cgpu_ctx* ctx);
+void cg_prefault(void* p, size_t bytes);
 // After the context stream is synchronised: CGPU_ERR_TIMEOUT (and a reset
 // count) if a traversal ran out of its device-side visit budget.
 cgpu_status cg_check_status(cgpu_ctx* ctx);

@@ -1330,6 +1330,7 @@ cgpu_status cg_render_paths_raw(cgpu_ctx* ctx, int scene, int mode, uint32_t fir
         st = run_batch(ctx, mode, sl.max_depth, k * npix, false, false);
         if (st != CGPU_OK) break;
         k_gather_paths<<<grid_for(ctx, k_gather_paths, 256, k * npix), 256, 0, ctx->stream>>>(ctx->wf.L, ctx->wf.Le, ctx->wf.Ls, k * npix, d_out);
+        cg_prefault(host_rgb + size_t(done) * npix * 3, size_t(k) * npix * 3 * sizeof(float));
         cudaMemcpyAsync(host_rgb + size_t(done) * npix * 3, d_out, size_t(k) * npix * 3 * sizeof(float),
                         cudaMemcpyDeviceToHost, ctx->stream);
         done += k;
@@ -1358,6 +1359,7 @@ cgpu_status cg_path_radiance(cgpu_ctx* ctx, int scene, int mode, const double* f
                                                                                                 d_keys, n, d_out);
         e = cudaGetLastError();
     }
+    if (e == cudaSuccess) cg_prefault(out_rgb, size_t(n) * 12);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out_rgb, d_out, size_t(n) * 12, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cudaFree(d_xy);
