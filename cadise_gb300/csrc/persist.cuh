@@ -146,13 +146,17 @@ CG_D void pray_prep(PRay<SPH>& r, float3 d) {
     if constexpr (SPH) r.d = d;
 }
 
-// One pass over the `n` rays of a queue.  fetch(k, &o, &d, &tmax, &scene)
+// One pass over the `n` rays of a queue.  fetch(k, &o, &d, &tmin, &tmax, &scene)
 // loads entry k and returns the caller's id of the ray; finish(done, id, t,
 // slot, tie) is called by the whole warp with the lanes whose ray is done
 // (slot < 0: a miss; tie: two candidates within the tie window);
 // exhausted(id): the ray ran out of its visit budget.
-template <bool ANY, bool COUNT, bool SPH, class Fetch, class Finish, class Exhausted>
-CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, float tmin, Fetch&& fetch, Finish&& finish,
+// GENERAL (ray queries): every ray has its own tmin, and closest-hit rays cull
+// nodes by the tie window's far end, so that every primitive within the window
+// is met; the render's rays all start at kRayEps and cull by the hit itself
+// (4 % faster; ties are then found where both primitives are met).
+template <bool ANY, bool COUNT, bool SPH, bool GENERAL, class Fetch, class Finish, class Exhausted>
+CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fetch&& fetch, Finish&& finish,
                           Exhausted&& exhausted, TraceCounters& tc) {
     PStack<!ANY> stack;
     uint32_t over[PStack<!ANY>::kOver * (ANY ? 1 : 2)];  // the entries beyond the shared rows
@@ -161,7 +165,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, fl
     const Bvh4Node* nodes = nullptr;
     const TriRecord* tris = nullptr;
     float tie_abs = 0.0f;
-    float tcur = 0.0f;
+    float tcur = 0.0f, ray_tmin = 0.0f;
     int hslot = -1;
     bool tie = false;
     int left = 0;        // node and leaf visits left, negative once the budget is exceeded
@@ -192,7 +196,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, fl
                 float3 d;
                 int scene = 0;
                 tcur = kFloatMax;
-                p = fetch(pool + rank, &r.o, &d, &tcur, &scene);
+                p = fetch(pool + rank, &r.o, &d, &ray_tmin, &tcur, &scene);
                 const SceneD* S = scenes + scene;
                 nodes = S->nodes;
                 tris = S->tris;
@@ -211,6 +215,8 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, fl
         if (need == kFullWarp) break;
         // ---- steps
         for (int round = kRoundSteps - 1;;) {
+            const float tmin = GENERAL ? ray_tmin : kRayEps;
+            const float tcull = GENERAL && !ANY ? tcur * kTieSlack + tie_abs : tcur;
             // a leaf is postponed (once); a lane without a node takes its next
             // stack entry (one a step: a culled one costs it the step)
             if (cur < -1 && leaf == -1) {
@@ -239,7 +245,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, fl
                     "setp.le.and.f32 q, t, %3, p;\n\t"
                     "@q mov.b32 %0, e;\n\t}"
                     : "+r"(cur), "+r"(stack.sp)
-                    : "r"(stack.base), "f"(tcur * kBoxSlack));
+                    : "r"(stack.base), "f"(tcull * kBoxSlack));
             }
             if (cur < -1 && leaf == -1) {
                 leaf = cur;
@@ -265,7 +271,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, fl
                     load_node(nodes, uint32_t(cur), nd);
                     if (COUNT) tc.nodes++;
                     float tn[4];
-                    child_hits(r.o, r.inv, tmin, nd, tcur, tn);
+                    child_hits(r.o, r.inv, tmin, nd, tcull, tn);
                     const uint32_t ce[4] = {__float_as_uint(nd[1].x), __float_as_uint(nd[1].y),
                                             __float_as_uint(nd[1].z), __float_as_uint(nd[1].w)};
                     // room for the three children a visit may push

@@ -111,3 +111,41 @@ def test_tiny_queues_match_the_megakernel(gpu_ctx, w, h):
         gpu_ctx.release(sid)
     for x, y in zip(*films):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["field", "features", "spheres", "coplanar", "shells"])
+def test_query_batches_match_small_queries(gpu_ctx, name):
+    """A batch that goes through the persistent pass gives the answers of the
+    same rays asked in pieces that do not: random rays, rays with their own
+    (also negative) t_min and short t_max, zero direction components,
+    unnormalised directions, rays that start on a surface."""
+    from golden_scenes import specs
+    spec = shells(700) if name == "shells" else specs()[name]
+    sid = gpu_ctx.upload(abi.flatten(spec))
+    info = gpu_ctx.info(sid)
+    lo, hi = np.array(info.bounds_min), np.array(info.bounds_max)
+    rng = np.random.default_rng(9)
+    n = (1 << 17) + 33
+    size = np.linalg.norm(hi - lo)
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, :3] = lo - 0.1 * (hi - lo) + 1.2 * (hi - lo) * rng.random((n, 3))
+    rays[:, 4:7] = rng.normal(0, 1, (n, 3)) * rng.uniform(0.1, 10, (n, 1))
+    rays[:, 3] = 1e-3
+    rays[:, 7] = 3.4e38
+    k = n // 8
+    rays[:k, 3] = rng.uniform(-0.5, 0.5, k) * size
+    rays[k:2 * k, 7] = rng.uniform(0, 0.3, k) * size
+    rays[2 * k:3 * k, 4 + rng.integers(0, 3)] = 0.0
+    rays[3 * k:4 * k, 4] = -0.0
+    rays[3 * k:4 * k, 5] = 0.0
+    prim, t, _, _ = gpu_ctx.trace_closest(sid, rays[4 * k:5 * k])
+    d = rays[4 * k:5 * k, 4:7] / np.linalg.norm(rays[4 * k:5 * k, 4:7], axis=1, keepdims=True)
+    rays[5 * k:6 * k, :3] = rays[4 * k:5 * k, :3] + d * t[:, None]  # (misses: their own origin)
+    whole = gpu_ctx.trace_closest(sid, rays), (gpu_ctx.trace_any(sid, rays),)
+    parts = [(gpu_ctx.trace_closest(sid, rays[i:i + 1000]), (gpu_ctx.trace_any(sid, rays[i:i + 1000]),))
+             for i in range(0, n, 1000)]
+    for q in (0, 1):
+        for j in range(len(whole[q])):
+            assert np.array_equal(whole[q][j], np.concatenate([p[q][j] for p in parts])), (name, q, j)
+    gpu_ctx.release(sid)
