@@ -41,7 +41,7 @@ struct FilmD {
 };
 
 // Counters per bounce b at cnt[b * kCntStride + k]:
-//   k = 0 continuation rays to extend, 1 MIS rays to extend, 2 shadow rays,
+//   k = 0 continuation rays to extend, 1 unused, 2 shadow rays,
 //   3 + kind: hits waiting for the shade kernel of that BSDF kind,
 //   8 / 9: rays handed out so far by the persistent extend / shadow kernels,
 //   10: adjoint vertices of bounce b - 1 (the wavefront adjoint's gradient kernel),
@@ -68,8 +68,7 @@ struct WfBuffers {
     int* q_mocc[2];   // MIS occlusion queries, ping-pong on the bounce
     int* q_mat[kNumBsdfKinds];
     // closest-hit rays whose persistent traversal met two primitives within
-    // the tie window (k_wf_extend_pww), for k_wf_ties: path, | 0x80000000 for
-    // a MIS ray; room for every ray of a pass (2 per path)
+    // the tie window (k_wf_extend_pww), for k_wf_ties: paths
     int* q_tie;
     int* cnt;
     int cnt_depth;    // bounces the counter array covers
@@ -181,7 +180,7 @@ struct RenderArgs {
     WfBuffers wf;
     unsigned long long* counters;  // closest rays, any rays, nodes, tris, paths
     AdjBufs adj;      // wavefront adjoint only
-    // reordered closest-hit queue (tuning.reorder): path | 0x80000000 for a MIS ray
+    // reordered closest-hit queue (tuning.reorder): paths
     const uint32_t* sorted;
     // persistent traversal passes: a warp refills its finished lanes once
     // fewer than this many of its lanes still trace (cgpu_tuning)

@@ -49,6 +49,8 @@ constexpr int kSmemStack = 16, kSpill = 8;
 // the dynamic shared memory of a persistent traversal launch
 extern __shared__ __align__(16) uint32_t trav_stack_smem[];
 
+constexpr int kSlotMask = int(kMaxTriSlots);
+
 // Shared memory of a block of `threads` threads.
 constexpr CG_HD uint32_t persist_warp_bytes(bool with_t) { return uint32_t(kSmemStack) * 32u * (with_t ? 8u : 4u); }
 constexpr size_t persist_bytes(int threads, bool with_t) { return size_t(threads / 32) * persist_warp_bytes(with_t); }
@@ -148,8 +150,8 @@ CG_D void pray_prep(PRay<SPH>& r, float3 d) {
 
 // One pass over the `n` rays of a queue.  fetch(k, &o, &d, &tmin, &tmax, &scene)
 // loads entry k and returns the caller's id of the ray; finish(done, id, t,
-// slot, tie) is called by the whole warp with the lanes whose ray is done
-// (slot < 0: a miss; tie: two candidates within the tie window);
+// slot, kind, tie) is called by the whole warp with the lanes whose ray is done
+// (slot < 0: a miss; kind: the record's shade queue; tie: two candidates within the tie window);
 // exhausted(id): the ray ran out of its visit budget.
 // GENERAL (ray queries): every ray has its own tmin, and closest-hit rays cull
 // nodes by the tie window's far end, so that every primitive within the window
@@ -355,8 +357,9 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                         stack.clear();
                     } else {
                         if (hslot >= 0 && t * kTieSlack + tie_abs >= tcur) tie = true;
-                        if (hslot < 0 ? t <= tcur : (t < tcur || (t == tcur && int(slot) < hslot))) {
-                            hslot = int(slot);
+                        if (hslot < 0 ? t <= tcur : (t < tcur || (t == tcur && int(slot) < (hslot & kSlotMask)))) {
+                            // the record's shade queue rides above its 28 slot bits
+                            hslot = int(slot | (__float_as_uint(c.w) >> kRecQueueShift << 28));
                             tcur = t;
                         }
                     }
@@ -372,7 +375,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
         const bool over = left < 0 || (left == 0 && cur >= 0);
         const bool done = p >= 0 && (over || (cur == -1 && leaf == -1 && stack.sp == stack.base));
         if (done && over) exhausted(p);
-        finish(done, p, tcur, hslot, tie);
+        finish(done, p, tcur, hslot < 0 ? -1 : hslot & kSlotMask, hslot >> 28, tie);
         if (done) {
             p = -1;
             cur = leaf = -1;

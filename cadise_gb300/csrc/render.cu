@@ -104,68 +104,33 @@ CG_D void grouped_push(int* const* queues, int* counters, int key, int p) {
     if (key >= 0) queues[key][base + __popc(grp & ((1u << lane) - 1u))] = p;
 }
 
-// After a closest-hit trace of queue entry p: a continuation hit is stored
-// and its BSDF kind returned (the shade queue to join); an escaped
-// continuation ray picks up the sky; a MIS ray that reaches its light adds
-// the BSDF-sampling half of the NEE estimate.  Returns -1 when nothing is
-// queued.
-// ADJ (wavefront adjoint): the MIS half and its derivative by the light's
-// radiance go to adj.mis_B / mis_X instead of L.
-template <bool ADJ = false>
-CG_D int extend_finish(const WfBuffers& w, const SceneD& S, int p, bool cont, float3 o, float3 d, bool hitp,
-                       const HitD& hit, const AdjBufs* adj = nullptr) {
-    if (cont) {
-        if (hitp) {
-            __stcs(&w.hit[p], make_float4(hit.t, __int_as_float(hit.slot), hit.u, hit.v));
-            return shade_queue(S.materials[material_of_slot(S, hit.slot)].type);
+// After the closest-hit trace of path p's continuation ray: a hit is stored
+// and its path joins the shade queue of the material; an escaped ray picks up
+// the sky.  The queue comes with the record (kind), not by way of the
+// material table: two dependent loads less at the few lanes that finish
+// together (closest-hit passes of the 1 M-triangle frame 34.5 -> 34.2 ms).
+CG_D void extend_finish(const WfBuffers& w, const SceneD& S, int* counters, int p, float t, int slot, int kind) {
+    if (slot >= 0) {
+        __stcs(&w.hit[p], make_float4(t, __int_as_float(slot), 0.0f, 0.0f));
+    } else if (S.env_light >= 0) {
+        const float4 tw = w.thr[p];
+        if (__float_as_int(tw.w) & 1) {
+            const float3 e = f3(tw) * env_radiance(S, f3(w.ray_d[p]));
+            w.Le[p] = make_float4(e.x, e.y, e.z, 0.0f);
         }
-        if (S.env_light >= 0) {
-            const float4 tw = w.thr[p];
-            if (__float_as_int(tw.w) & 1) {
-                const float3 e = f3(tw) * env_radiance(S, d);
-                w.Le[p] = make_float4(e.x, e.y, e.z, 0.0f);
-            }
-        }
-        return -1;
     }
-    const float4 mb = w.mis_b[p];
-    const int mlight = __float_as_int(mb.w);
-    float3 add = splat3(0.0f), X = splat3(0.0f);
-    bool has = false;
-    int xlight = -1;
-    if (hitp) {
-        if (light_of_slot(S, hit.slot) == mlight) {
-            const SurfaceD hs = surface_at(S, o, d, hit);
-            const float4 ma = w.mis_a[p];
-            add = mis_resolve(S, hs, o, f3(mb), f3(ma), ma.w, ADJ ? &X : nullptr);
-            has = true;
-            xlight = mlight;
-        }
-    } else if (mlight == S.env_light) {
-        const float4 ma = w.mis_a[p];
-        add = mis_resolve_env(S, d, f3(mb), f3(ma), ma.w);
-        has = true;
-    }
-    if (ADJ) {
-        if (has) {
-            adj->mis_B[p] = make_float4(add.x, add.y, add.z, 1.0f);
-            adj->mis_X[p] = make_float4(X.x, X.y, X.z, __int_as_float(xlight));
-        }
-        return -1;
-    }
-    if (has) {
-        float4 L = w.L[p];
-        L.x += add.x;
-        L.y += add.y;
-        L.z += add.z;
-        w.L[p] = L;
-    }
-    return -1;
+    grouped_push(w.q_mat, counters, kind, p);
+}
+
+// The shade queue of a record's material.
+CG_D int kind_of_slot(const SceneD& S, int slot) {
+    return slot < 0 ? -1 : int(__float_as_uint(ldg4(reinterpret_cast<const float4*>(S.tris + slot) + 2).w) >> kRecQueueShift);
 }
 
 // MIS rays that meet their light (mis_light_hit): unless a primitive comes
-// before the light's hit, the MIS term of extend_finish, added to L (ADJ:
-// stored with its radiance derivative for the adjoint's gradient kernel).
+// before the light's hit, the BSDF-sampling half of the NEE estimate, added to
+// L (ADJ: stored with its radiance derivative for the adjoint's gradient
+// kernel).
 template <bool COUNT, bool SPH, bool ADJ = false>
 __global__ void k_wf_mis_occl(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
@@ -227,19 +192,6 @@ CG_D void shadow_finish(const WfBuffers& w, int p, bool occluded) {
     w.Ls[p] = Ls;
 }
 
-// Queue entry i of a closest-hit pass: its path and whether it is a
-// continuation ray (else a MIS ray); SORTED reads the reordered queue.
-template <bool SORTED>
-CG_D int extend_entry(const RenderArgs& a, const int* qc, const int* qm, int ncont, int i, bool* cont) {
-    if (SORTED) {
-        const uint32_t e = a.sorted[i];
-        *cont = (e >> 31) == 0u;
-        return int(e & 0x7FFFFFFFu);
-    }
-    *cont = i < ncont;
-    return *cont ? qc[i] : qm[i - ncont];
-}
-
 CG_D uint32_t spread9(uint32_t v) {
     uint32_t x = v & 0x1FFu;
     x = (x | (x << 16)) & 0x030000FFu;
@@ -252,20 +204,16 @@ CG_D uint32_t spread9(uint32_t v) {
 // Sort keys of a closest-hit pass's queue (tuning.reorder): the direction's
 // octant above the Morton code of the origin in the scene bounds (`bits` per
 // axis, at most 9), so that sorted neighbours leave nearby points in similar
-// directions.  Values: path | 0x80000000 for a MIS ray.  Writes the entry
-// count for the sort.
+// directions.  Values: paths.  Writes the entry count for the sort.
 __global__ void k_ray_keys(RenderArgs a, int b, int bits, uint32_t* keys, uint32_t* vals, uint32_t* n_out) {
     const WfBuffers& w = a.wf;
     const int* cnt = w.cnt + b * kCntStride;
-    const int ncont = cnt[0], n = ncont + cnt[1];
+    const int n = cnt[0];
     const int* qc = w.q_cont[b & 1];
-    const int* qm = w.q_mis[b & 1];
     if (blockIdx.x == 0 && threadIdx.x == 0) *n_out = uint32_t(n);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const bool cont = i < ncont;
-        const int p = cont ? qc[i] : qm[i - ncont];
-        const float3 o = f3(w.ray_o[p]);
-        const float3 d = cont ? f3(w.ray_d[p]) : f3(w.mis_d[p]);
+        const int p = qc[i];
+        const float3 o = f3(w.ray_o[p]), d = f3(w.ray_d[p]);
         const SceneD& S = a.scenes[w.meta[p].x];
         const float u[3] = {(o.x - S.bounds_lo.x) * S.bounds_inv.x, (o.y - S.bounds_lo.y) * S.bounds_inv.y,
                             (o.z - S.bounds_lo.z) * S.bounds_inv.z};
@@ -274,33 +222,26 @@ __global__ void k_ray_keys(RenderArgs a, int b, int bits, uint32_t* keys, uint32
         for (int k = 0; k < 3; ++k) q[k] = uint32_t(fminf(fmaxf(u[k], 0.0f), 1.0f) * cells);
         const uint32_t oct = (d.x < 0.0f ? 4u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 1u : 0u);
         keys[i] = (oct << (3 * bits)) | (spread9(q[0]) << 2) | (spread9(q[1]) << 1) | spread9(q[2]);
-        vals[i] = uint32_t(p) | (cont ? 0u : 0x80000000u);
+        vals[i] = uint32_t(p);
     }
 }
 
-template <bool COUNT, bool SPH, bool ADJ = false, bool SORTED = false>
+template <bool COUNT, bool SPH, bool SORTED = false>
 __global__ void k_wf_extend(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
     int* cnt = w.cnt + b * kCntStride;
-    const int ncont = cnt[0], nmis = cnt[1];
-    const int n = ncont + nmis;
-    const int* qc = w.q_cont[b & 1];
-    const int* qm = w.q_mis[b & 1];
+    const int n = cnt[0];
+    const int* q = SORTED ? reinterpret_cast<const int*>(a.sorted) : w.q_cont[b & 1];
     TraceCounters tc{0, 0};
     uint32_t nclosest = 0;
-    int* const* qmat = w.q_mat;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        bool cont;
-        const int p = extend_entry<SORTED>(a, qc, qm, ncont, i, &cont);
+        const int p = q[i];
         const SceneD& S = a.scenes[w.meta[p].x];
-        const float3 o = f3(w.ray_o[p]);
-        const float3 d = cont ? f3(w.ray_d[p]) : f3(w.mis_d[p]);
-        const RayPre r = ray_prep(o, d, kRayEps, kFloatMax);
+        const RayPre r = ray_prep(f3(w.ray_o[p]), f3(w.ray_d[p]), kRayEps, kFloatMax);
         HitD hit;
         if (COUNT) ++nclosest;
-        const bool hitp = traverse_warp<COUNT, SPH>(S, r, &hit, &tc);
-        const int key = extend_finish<ADJ>(w, S, p, cont, o, d, hitp, hit, &a.adj);
-        grouped_push(qmat, cnt + 3, key, p);
+        if (!traverse_warp<COUNT, SPH>(S, r, &hit, &tc)) hit.slot = -1;
+        extend_finish(w, S, cnt + 3, p, hit.t, hit.slot, kind_of_slot(S, hit.slot));
     }
     count_flush<COUNT>(a.counters, tc, TraceCounters{0, 0}, nclosest, 0);
 }
@@ -349,18 +290,14 @@ template <bool COUNT, bool SPH>
 __global__ void k_wf_extend_dyn(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
     int* cnt = w.cnt + b * kCntStride;
-    const int ncont = cnt[0], nmis = cnt[1];
-    const int n = ncont + nmis;
-    const int* qc = w.q_cont[b & 1];
-    const int* qm = w.q_mis[b & 1];
+    const int n = cnt[0];
+    const int* q = w.q_cont[b & 1];
     TraceCounters tc{0, 0};
     uint32_t nclosest = 0;
-    int* const* qmat = w.q_mat;
     TravState st;
     RayPre r;
     int i = -1, p = -1;
     bool drained = false;
-    float3 o = splat3(0.0f), d = splat3(0.0f);
     for (;;) {
         const bool need = i < 0 && !drained;
         const int k = warp_take(cnt + 8, need, n);
@@ -369,11 +306,8 @@ __global__ void k_wf_extend_dyn(RenderArgs a, int b) {
                 drained = true;
             } else {
                 i = k;
-                const bool cont = i < ncont;
-                p = cont ? qc[i] : qm[i - ncont];
-                o = f3(w.ray_o[p]);
-                d = cont ? f3(w.ray_d[p]) : f3(w.mis_d[p]);
-                r = ray_prep(o, d, kRayEps, kFloatMax);
+                p = q[i];
+                r = ray_prep(f3(w.ray_o[p]), f3(w.ray_d[p]), kRayEps, kFloatMax);
                 trav_begin(st, r, a.scenes[w.meta[p].x].visit_budget);
                 if (COUNT) ++nclosest;
             }
@@ -383,13 +317,7 @@ __global__ void k_wf_extend_dyn(RenderArgs a, int b) {
             const SceneD& S = a.scenes[w.meta[p].x];
             for (int s = 0; s < kStepsPerFetch && !st.done; ++s) trav_step<false, COUNT, SPH>(S, r, st, &tc);
             if (st.done) {
-                HitD hit;
-                hit.slot = st.hslot;
-                hit.t = st.tcur;
-                hit.u = st.hu;
-                hit.v = st.hv;
-                const int key = extend_finish(w, S, p, i < ncont, o, d, st.hslot >= 0, hit);
-                grouped_push(qmat, cnt + 3, key, p);
+                extend_finish(w, S, cnt + 3, p, st.tcur, st.hslot, kind_of_slot(S, st.hslot));
                 i = -1;
             }
         }
@@ -404,19 +332,18 @@ constexpr int kPersistRegs = 56;
 
 // Persistent closest-hit pass (persist.cuh) over the continuation rays.  A ray
 // that meets two primitives within the tie window is left to k_wf_ties.
-template <bool COUNT, bool SPH, bool SORTED = false, bool ADJ = false>
+template <bool COUNT, bool SPH, bool SORTED = false>
 __global__ void __maxnreg__(kPersistRegs) k_wf_extend_pww(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
     int* cnt = w.cnt + b * kCntStride;
     const int n = cnt[0];
-    const int* qc = w.q_cont[b & 1];
+    const int* q = SORTED ? reinterpret_cast<const int*>(a.sorted) : w.q_cont[b & 1];
     TraceCounters tc{0, 0};
     uint32_t nclosest = 0;
     persistent_pass<false, COUNT, SPH, false>(
         a.scenes, cnt + 8, n, a.refill_closest,
         [&](int k, float3* o, float3* d, float*, float* tmax, int* scene) {
-            bool cont;
-            const int p = extend_entry<SORTED>(a, qc, nullptr, n, k, &cont);
+            const int p = q[k];
             *o = f3(__ldcs(&w.ray_o[p]));
             *d = f3(__ldcs(&w.ray_d[p]));
             *scene = int(__ldcs(&w.meta[p].x));
@@ -424,22 +351,10 @@ __global__ void __maxnreg__(kPersistRegs) k_wf_extend_pww(RenderArgs a, int b) {
             if (COUNT) ++nclosest;
             return p;
         },
-        [&](bool done, int p, float t, int slot, bool tie) {
+        [&](bool done, int p, float t, int slot, int kind, bool tie) {
             if (!done) return;
-            if (tie) {
-                w.q_tie[atomicAdd(cnt + 12, 1)] = p;
-            } else {
-                HitD hit;
-                hit.t = t;
-                hit.slot = slot;
-                hit.u = 0.0f;
-                hit.v = 0.0f;
-                const SceneD& S = a.scenes[__ldcs(&w.meta[p].x)];
-                const float3 o = splat3(0.0f);
-                const float3 d = S.env_light >= 0 ? f3(__ldcs(&w.ray_d[p])) : splat3(0.0f);
-                const int key = extend_finish<ADJ>(w, S, p, true, o, d, slot >= 0, hit, &a.adj);
-                grouped_push(w.q_mat, cnt + 3, key, p);
-            }
+            if (tie) w.q_tie[atomicAdd(cnt + 12, 1)] = p;
+            else extend_finish(w, a.scenes[__ldcs(&w.meta[p].x)], cnt + 3, p, t, slot, kind);
         },
         [&](int p) {
             uint32_t* st = a.scenes[w.meta[p].x].status;
@@ -457,29 +372,21 @@ constexpr int kTieBlock = 64;
 // traversal (closer_hit / tie_prefers, wide culling), then finished as the
 // persistent pass finishes its other rays.  It runs beside the any-hit pass
 // (on the other stream), and its grid strides over however few rays it got.
-template <bool COUNT, bool SPH, bool ADJ = false>
+template <bool COUNT, bool SPH>
 __global__ void k_wf_ties(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
     int* cnt = w.cnt + b * kCntStride;
     const int n = cnt[12];
-    int* const* qmat = w.q_mat;
     TraceCounters tc{0, 0};
     uint32_t nties = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (COUNT) ++nties;
-        const int e = w.q_tie[i];
-        const bool cont = e >= 0;
-        const int p = e & 0x7FFFFFFF;
+        const int p = w.q_tie[i];
         const SceneD& S = a.scenes[w.meta[p].x];
-        const float3 o = f3(w.ray_o[p]);
-        const float3 d = cont ? f3(w.ray_d[p]) : f3(w.mis_d[p]);
-        const RayPre r = ray_prep(o, d, kRayEps, kFloatMax);
+        const RayPre r = ray_prep(f3(w.ray_o[p]), f3(w.ray_d[p]), kRayEps, kFloatMax);
         HitD hit;
-        const bool hitp = traverse<false, COUNT, SPH>(S, r, &hit, &tc);
-        hit.u = 0.0f;
-        hit.v = 0.0f;
-        const int key = extend_finish<ADJ>(w, S, p, cont, o, d, hitp, hit, &a.adj);
-        grouped_push(qmat, cnt + 3, key, p);
+        if (!traverse<false, COUNT, SPH>(S, r, &hit, &tc)) hit.slot = -1;
+        extend_finish(w, S, cnt + 3, p, hit.t, hit.slot, kind_of_slot(S, hit.slot));
     }
     count_flush<COUNT>(a.counters, tc, TraceCounters{0, 0}, 0, 0);
     if (COUNT && nties) atomicAdd(a.counters + 6, (unsigned long long)nties);
@@ -507,7 +414,7 @@ __global__ void __maxnreg__(kPersistRegs) k_wf_shadow_pww(RenderArgs a, int b) {
             if (COUNT) ++nany;
             return p;
         },
-        [&](bool done, int p, float, int slot, bool) {
+        [&](bool done, int p, float, int slot, int, bool) {
             if (done) shadow_finish<ADJ>(w, p, slot >= 0);
         },
         [&](int p) {
@@ -907,7 +814,7 @@ __global__ void __maxnreg__(kPersistRegs) k_query(const SceneD* scenes, int scen
             *s = scene;
             return k;
         },
-        [&](bool done, int k, float t, int slot, bool tie) {
+        [&](bool done, int k, float t, int slot, int, bool tie) {
             if (!done) return;
             if (ANY) {
                 occ[k] = slot >= 0 ? 1 : 0;
@@ -1117,7 +1024,7 @@ cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool spl
 #undef CG_PICK
     // reordered closest-hit passes after the first (the primary rays are in pixel order already)
     const bool reorder = ctx->tuning.reorder != 0 && trav != 1 && ctx->sort_block != nullptr;
-#define CG_PICK_SORTED(C, S) (trav >= 2 ? k_wf_extend_pww<C, S, true> : k_wf_extend<C, S, false, true>)
+#define CG_PICK_SORTED(C, S) (trav >= 2 ? k_wf_extend_pww<C, S, true> : k_wf_extend<C, S, true>)
     auto ext_sorted = sph ? (counting ? CG_PICK_SORTED(true, true) : CG_PICK_SORTED(false, true))
                           : (counting ? CG_PICK_SORTED(true, false) : CG_PICK_SORTED(false, false));
 #undef CG_PICK_SORTED
@@ -1505,12 +1412,12 @@ void enqueue_adjoint_pass(cgpu_ctx* ctx, const RenderArgs& a, int depth, uint32_
     const bool sph = ctx->batch_spheres;
     // the persistent passes when the tuning uses them (traversal 2 / 3), else the per-ray loops
     const int trav = ctx->tuning.traversal;
-    auto ext = trav >= 2 ? (sph ? k_wf_extend_pww<false, true, false, true> : k_wf_extend_pww<false, false, false, true>)
-                         : (sph ? k_wf_extend<false, true, true> : k_wf_extend<false, false, true>);
+    auto ext = trav >= 2 ? (sph ? k_wf_extend_pww<false, true> : k_wf_extend_pww<false, false>)
+                         : (sph ? k_wf_extend<false, true> : k_wf_extend<false, false>);
     auto shd = trav == 3 ? (sph ? k_wf_shadow_pww<false, true, true> : k_wf_shadow_pww<false, false, true>)
                          : (sph ? k_wf_shadow<false, true, true> : k_wf_shadow<false, false, true>);
     auto mo = sph ? k_wf_mis_occl<false, true, true> : k_wf_mis_occl<false, false, true>;
-    auto ties = sph ? k_wf_ties<false, true, true> : k_wf_ties<false, false, true>;
+    auto ties = sph ? k_wf_ties<false, true> : k_wf_ties<false, false>;
     void (*shade[kNumBsdfKinds])(RenderArgs, int) = {k_wf_shade<0, true>, k_wf_shade<1, true>, k_wf_shade<2, true>,
                                                      k_wf_shade<3, true>, k_wf_shade<4, true>};
     k_wf_generate<<<grid_for(ctx, k_wf_generate, kBlock, paths), kBlock, 0, s>>>(a);

@@ -213,7 +213,8 @@ cgpu_status build_host_scene(const cgpu_scene_desc* d, HostScene* out, std::stri
         }
         std::memcpy(&R.v0.w, &prim, 4);
         std::memcpy(&R.v1.w, &packed, 4);
-        std::memcpy(&R.v2.w, &tflags[t], 4);
+        const uint32_t flags = tflags[t] | uint32_t(shade_queue(d->materials[mat].type)) << kRecQueueShift;
+        std::memcpy(&R.v2.w, &flags, 4);
     }
     // rect flags carry the rectangle index; the device reads frames by it
     // ---- materials

@@ -102,7 +102,7 @@ constexpr int kStackSize = 96;
 struct __align__(16) TriRecord {
     float4 v0;  // xyz = vertex A, w = primitive index (int bits)
     float4 v1;  // xyz = vertex B, w = (material index) | ((light index + 1) << 16)
-    float4 v2;  // xyz = vertex C, w = flags (kRec* kind in bits 0-1, rectangle index in bits 2-31)
+    float4 v2;  // xyz = vertex C, w = flags (kRec* below)
     // a sphere: v0.xyz = centre, v1.x = radius
 };
 static_assert(sizeof(TriRecord) == 48, "TriRecord is 48 bytes");
@@ -128,8 +128,11 @@ constexpr CG_HD int shade_queue(int type) {
 template <int Q>
 constexpr CG_HD bool queue_has(int type) { return Q < 0 || shade_queue(type) == Q; }
 
-// Record flags (TriRecord::v2.w): bits 0-1 the kind, bits 2-31 the
-// rectangle index of a rectangle half.
+// Record flags (TriRecord::v2.w): bits 0-1 the kind, bits 2-28 the rectangle
+// index of a rectangle half (two records each, so below kMaxTriSlots / 2),
+// bits 29-31 the shade queue of the material.
+constexpr int kRecQueueShift = 29;
+CG_HD uint32_t rec_rect(uint32_t flags) { return (flags >> 2) & 0x07FFFFFFu; }
 constexpr uint32_t kRecTriangle = 0u, kRecRectHalf = 1u, kRecSphere = 2u;
 
 struct __align__(16) MaterialD {

@@ -131,7 +131,7 @@ CG_D HitPoint hit_point(const SceneD& S, float3 o, float3 d, const HitD& h) {
         return hp;
     }
     if ((flags & 3u) == kRecRectHalf) {
-        hp.rect = int(flags >> 2);
+        hp.rect = int(rec_rect(flags));
         float3 vB, eA, eB;
         rect_frame(S, hp.rect, &vB, &eA, &eB);
         hp.t = ref_rect_t(o, d, vB, eA, eB, h.t);

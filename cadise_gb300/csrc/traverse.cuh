@@ -329,7 +329,7 @@ CG_D bool ref_hit(const SceneD& S, const RayPre& r, int slot, float* tout) {
     const uint32_t flags = __float_as_uint(c.w);
     if ((flags & 3u) == kRecSphere) return sphere_test(r, f3(a), b.x, r.tmax, tout);
     if ((flags & 3u) == kRecRectHalf) {
-        const float* fr = S.rect_frames + 9 * size_t(flags >> 2);
+        const float* fr = S.rect_frames + 9 * size_t(rec_rect(flags));
         const float3 vB = mk(fr[0], fr[1], fr[2]), eA0 = mk(fr[3], fr[4], fr[5]), eB0 = mk(fr[6], fr[7], fr[8]);
         float3 eA = eA0, eB = eB0;
         if (dot(r.d, cross(eA, eB)) > 0.0f) {
