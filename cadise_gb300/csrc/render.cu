@@ -608,8 +608,15 @@ __global__ void k_adj_ltot(RenderArgs a) {
     }
 }
 
+// Bound by latency (long scoreboard, 20 resident warps an SM) and by
+// instruction fetch: one kernel over all kinds, grouped in shared memory, took
+// 39 to 135 ms where these five take 14.9 (1 M-triangle frame, 16 samples a
+// pixel).  96 registers keep five blocks of 128 threads on an SM: 14.9 ms,
+// 15.8 uncapped (up to 115 registers), 15.6 at 80, 17.1 at 64.
+constexpr int kShadeRegs = 96;
+
 template <int KIND, bool ADJ = false>
-__global__ void k_wf_shade(RenderArgs a, int b) {
+__global__ void __maxnreg__(kShadeRegs) k_wf_shade(RenderArgs a, int b) {
     extern __shared__ double adj_sh[];  // ADJ only: gradient block sums
     const WfBuffers& w = a.wf;
     const int n = w.cnt[b * kCntStride + 3 + KIND];
