@@ -51,9 +51,27 @@ CG_HD void footprint_1d(float p, float half, int t0, int t1, int* a, int* b) {
     *b = int(floorf(hi - 0.5f) + 1.0f);
 }
 
-// How far (in pixels) a sample's footprint can reach from its own pixel, with
-// one pixel of margin for the rounding of the bounds.
-CG_HD int footprint_reach(float half) { return int(ceilf(half + 0.5f)) + 1; }
+// How far (in pixels) a sample's footprint can reach from its own pixel on an
+// axis of `extent` pixels: a sample lies within its pixel, so floor(half + 1/2),
+// with the roundings of two FP32 sums of coordinates up to the extent.  (One
+// and two pixels more, as a margin, made the gather of a 4-pixel filter look at
+// 81 source pixels instead of 25: sphere box, 333 x 251, 9 samples, 1.28 ->
+// 0.68 ms with filter_add's fused sums.)
+CG_HD int footprint_reach(float half, int extent) { return int(floorf(half + 0.5f + 0.001f + float(extent) * 4e-7f)); }
+
+// One sample's contribution.  FP64 operations bound the gather (about 1.5 a clock
+// and SM), so the square's last product joins its sum in one of them; w v is
+// exact in FP64.
+CG_HD void filter_add(float3 v, float w, double* s, double* q, double* n) {
+    const double dw = w;
+    s[0] += double(v.x * w);
+    s[1] += double(v.y * w);
+    s[2] += double(v.z * w);
+    q[0] = fma(dw * v.x, double(v.x), q[0]);
+    q[1] = fma(dw * v.y, double(v.y), q[1]);
+    q[2] = fma(dw * v.z, double(v.z), q[2]);
+    *n += dw;
+}
 
 // Gather form of the footprint rule, for one pixel (ix, iy) of a W x H film:
 // the samples of the pixels of its own tile whose footprint covers it, in a
@@ -65,7 +83,7 @@ CG_HD void filter_gather(const FilterD& F, int W, int H, int ix, int iy, uint32_
                          double* q, double* n) {
     const int tx0 = ix / F.tile_w * F.tile_w, ty0 = iy / F.tile_h * F.tile_h;
     const int tx1 = min(tx0 + F.tile_w, W), ty1 = min(ty0 + F.tile_h, H);
-    const int rx = footprint_reach(F.hx), ry = footprint_reach(F.hy);
+    const int rx = footprint_reach(F.hx, W), ry = footprint_reach(F.hy, H);
     const int sx0 = max(tx0, ix - rx), sx1 = min(tx1 - 1, ix + rx);
     const int sy0 = max(ty0, iy - ry), sy1 = min(ty1 - 1, iy + ry);
     for (int sy = sy0; sy <= sy1; ++sy)
@@ -79,13 +97,7 @@ CG_HD void filter_gather(const FilterD& F, int W, int H, int ix, int iy, uint32_
                 footprint_1d(pos.y, F.hy, ty0, ty1, &ya, &yb);
                 if (ix < xa || ix >= xb || iy < ya || iy >= yb) continue;
                 const float w = filter_weight(F, float(ix) - (pos.x - 0.5f), float(iy) - (pos.y - 0.5f));
-                s[0] += double(v.x * w);
-                s[1] += double(v.y * w);
-                s[2] += double(v.z * w);
-                q[0] += double(w) * v.x * v.x;
-                q[1] += double(w) * v.y * v.y;
-                q[2] += double(w) * v.z * v.z;
-                *n += double(w);
+                filter_add(v, w, s, q, n);
             }
 }
 
