@@ -219,6 +219,7 @@ struct SceneSlot {
     cg::FilmD film{};
     int width = 0, height = 0, spp = 1, max_depth = 1;
     bool has_spheres = false;  // renders of this scene use the kernels with the sphere test
+    uint32_t kinds = 0;        // bit k: a material of shade queue k
 };
 
 struct cgpu_ctx {
@@ -270,8 +271,10 @@ struct cgpu_ctx {
     int graph_depth = -1;
     uint32_t graph_paths = 0;
     bool graph_spheres = false;
+    uint32_t graph_kinds = 0;
     uint32_t graph_launches = 0;  // kernel launches one replay of the graph makes
     bool batch_spheres = false;  // a scene of the current render holds spheres
+    uint32_t batch_kinds = 0;    // the shade queues of the current render's scenes
 
     cgpu_render_stats stats{};
 
