@@ -266,6 +266,12 @@ struct cgpu_ctx {
     uint32_t* d_status = nullptr;
     uint32_t visit_budget = 0;
 
+    // pinned stage of small host queries and the status word; device buffer of
+    // larger ones (trace_host)
+    char* h_stage = nullptr;
+    void* query_block = nullptr;
+    size_t query_cap = 0;
+
     // captured wavefront graph
     cudaGraphExec_t graph = nullptr;
     int graph_depth = -1;
@@ -303,6 +309,7 @@ cgpu_status cg_fail(cgpu_ctx* ctx, cgpu_status s, const std::string& msg);
 cgpu_status cg_cuda(cgpu_ctx* ctx, cudaError_t e, const char* what);
 cgpu_status cg_sync_tables(cgpu_ctx* ctx);
 void cg_prefault(void* p, size_t bytes);
-// After the context stream is synchronised: CGPU_ERR_TIMEOUT (and a reset
-// count) if a traversal ran out of its device-side visit budget.
-cgpu_status cg_check_status(cgpu_ctx* ctx);
+// Waits for the context stream (an error is reported as `what`'s); then
+// CGPU_ERR_TIMEOUT (and a reset count) if a traversal ran out of its visit
+// budget.
+cgpu_status cg_check_status(cgpu_ctx* ctx, const char* what);

@@ -1395,7 +1395,9 @@ cgpu_status cg_trace(cgpu_ctx* ctx, int scene, const cgpu_ray* d_rays, uint32_t 
             k_query_resolve<<<grid_for(ctx, k_query_resolve, kBlock, n), kBlock, 0, ctx->stream>>>(ctx->d_scenes, scene, d_rays, n,
                                                                                                  d_hits);
     } else {
-        k_trace<<<grid_for(ctx, k_trace, kBlock, n), kBlock, 0, ctx->stream>>>(ctx->d_scenes, scene, d_rays, n,
+        // few rays: a warp per block, so that each has an SM's pipes and L1 to itself
+        const int block = n < uint32_t(ctx->num_sms) * kBlock ? 32 : kBlock;
+        k_trace<<<grid_for(ctx, k_trace, block, n), block, 0, ctx->stream>>>(ctx->d_scenes, scene, d_rays, n,
                                                                             any ? nullptr : d_hits, any ? d_occ : nullptr);
     }
     return cg_cuda(ctx, cudaGetLastError(), "trace launch");
