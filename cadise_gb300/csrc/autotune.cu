@@ -23,11 +23,7 @@ bool valid_tuning(const cgpu_tuning& t) {
 void apply(cgpu_ctx* ctx, const cgpu_tuning& t) {
     const bool realloc = t.max_paths != ctx->tuning.max_paths;
     ctx->tuning = t;
-    if (ctx->graph) {
-        cudaGraphExecDestroy(ctx->graph);
-        ctx->graph = nullptr;
-    }
-    ctx->graph_depth = -1;
+    cg_drop_graphs(ctx);
     if (realloc) cg_free_render_state(ctx);
 }
 

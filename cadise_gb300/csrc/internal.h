@@ -187,6 +187,21 @@ struct RenderArgs {
     int refill_closest, refill_any;
 };
 
+// Where the tuning leaves the traversal variant open (traversal 0), the
+// persistent passes take batches of kLargeBatch paths through scenes of
+// kSmallScene records or more, and any batch through kLargeScene records or more
+// (ms a frame of depth 8, one ray per thread / persistent: 2,457,600 paths
+// through 960 triangles 3.22 / 3.03, through 204,800 7.71 / 5.96; 12,288 paths
+// through 51,200 0.96 / 0.90, through 204,800 1.05 / 0.97).  Elsewhere the second
+// launch for the rays within the tie window costs what they save (Cornell box,
+// 36 triangles, 1,048,576 paths 1.20 / 1.24; 262,144 paths through 3,200
+// triangles 1.05 / 1.06; an adjoint iteration of 96,520 paths through 3,842
+// triangles 1.86 / 1.96).  The adjoint's passes, launched one by one, go by the
+// paths alone; the allocation-free render, on one stream, takes the any-hit pass
+// (1.09 / 1.05).
+constexpr int kSmallScene = 512, kLargeScene = 16384;
+constexpr uint64_t kLargeBatch = 1u << 19;
+
 // The refill thresholds of a tuning, 0 replaced by the default.
 constexpr int kDefaultRefillLanes = 24;
 inline int refill_lanes(int32_t v) { return v > 0 ? v : kDefaultRefillLanes; }
@@ -272,15 +287,18 @@ struct cgpu_ctx {
     void* query_block = nullptr;
     size_t query_cap = 0;
 
-    // captured wavefront graph
-    cudaGraphExec_t graph = nullptr;
-    int graph_depth = -1;
-    uint32_t graph_paths = 0;
-    bool graph_spheres = false;
-    uint32_t graph_kinds = 0;
-    uint32_t graph_launches = 0;  // kernel launches one replay of the graph makes
+    // captured wavefront graphs: of one ray per thread and of persistent passes
+    struct Graph {
+        cudaGraphExec_t exec = nullptr;
+        int depth = -1;
+        uint32_t paths = 0;
+        bool spheres = false;
+        uint32_t kinds = 0;
+        uint32_t launches = 0;  // kernel launches one replay makes
+    } graphs[2];
     bool batch_spheres = false;  // a scene of the current render holds spheres
     uint32_t batch_kinds = 0;    // the shade queues of the current render's scenes
+    int batch_closest = 0, batch_any = 0;  // its traversal variants (choose_traversal)
 
     cgpu_render_stats stats{};
 
@@ -303,6 +321,7 @@ cgpu_status cg_trace(cgpu_ctx* ctx, int scene, const cgpu_ray* d_rays, uint32_t 
 cgpu_status cg_camera(cgpu_ctx* ctx, int scene, const double* d_xy, uint32_t n, float* d_out);
 cgpu_status cg_film_clear(cgpu_ctx* ctx, int scene);
 void cg_free_render_state(cgpu_ctx* ctx);
+void cg_drop_graphs(cgpu_ctx* ctx);
 
 // implemented in api.cu
 cgpu_status cg_fail(cgpu_ctx* ctx, cgpu_status s, const std::string& msg);

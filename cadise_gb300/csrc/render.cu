@@ -1012,6 +1012,15 @@ void collect_profile(cgpu_ctx* ctx) {
     ctx->prof.clear();
 }
 
+// The traversal variants of the current render's passes: the tuning's, or where
+// it leaves them open the persistent ones if the caller may use them (below).
+void choose_traversal(cgpu_ctx* ctx, bool closest, bool any) {
+    const int t = ctx->tuning.traversal;
+    ctx->batch_closest = t == 0 && closest ? 3 : t;
+    ctx->batch_any = t == 0 && any ? 3 : t;
+}
+bool large_batch(const cgpu_ctx* ctx, uint64_t paths) { return std::min<uint64_t>(paths, ctx->path_cap) >= kLargeBatch; }
+
 // The shade kernels of the queues that the render's scenes have materials for.
 // An empty launch still costs 2 to 4 us between two passes (Cornell box, 256 x
 // 256, 16 samples, depth 6: 1.28 -> 1.20 ms without four of them a bounce).
@@ -1041,12 +1050,12 @@ cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool spl
     const int bt = ctx->tuning.block_trace, bs = ctx->tuning.block_shade;
     const int ggen = grid_for(ctx, k_wf_generate, kBlock, paths);
     timed(ctx, CGPU_KERNEL_GENERATE, s, [&] { k_wf_generate<<<ggen, kBlock, 0, s>>>(a); });
-    const int trav = ctx->tuning.traversal;
+    const int trav = ctx->batch_closest, trav_any = ctx->batch_any;
     const bool sph = ctx->batch_spheres;
 #define CG_PICK(K) (sph ? (counting ? K<true, true> : K<false, true>) : (counting ? K<true, false> : K<false, false>))
     auto ext_kernel = trav == 1 ? CG_PICK(k_wf_extend_dyn)
                       : (trav == 2 || trav == 3) ? CG_PICK(k_wf_extend_pww) : CG_PICK(k_wf_extend);
-    auto sh_kernel = trav == 1 ? CG_PICK(k_wf_shadow_dyn) : trav == 3 ? CG_PICK(k_wf_shadow_pww) : CG_PICK(k_wf_shadow);
+    auto sh_kernel = trav_any == 1 ? CG_PICK(k_wf_shadow_dyn) : trav_any == 3 ? CG_PICK(k_wf_shadow_pww) : CG_PICK(k_wf_shadow);
     auto mocc_kernel = CG_PICK(k_wf_mis_occl);
     auto ties_kernel = CG_PICK(k_wf_ties);
 #undef CG_PICK
@@ -1065,7 +1074,7 @@ cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool spl
     // the persistent passes keep the bottom of their traversal stacks in shared memory
     const size_t ext_sm = stack_smem(ext_kernel, trav >= 2, true, bt);
     const size_t ext_sorted_sm = stack_smem(ext_sorted, trav >= 2, true, bt);
-    const size_t sh_sm = stack_smem(sh_kernel, trav == 3, false, bt);
+    const size_t sh_sm = stack_smem(sh_kernel, trav_any == 3, false, bt);
     const int gext = grid_for(ctx, ext_kernel, bt, paths, ext_sm);
     const int gsh = grid_for(ctx, sh_kernel, bt, paths, sh_sm);
     const int gmo = grid_for(ctx, mocc_kernel, bt, paths);
@@ -1138,12 +1147,14 @@ cgpu_status run_batch(cgpu_ctx* ctx, int mode, int depth, uint32_t paths, bool s
         return cg_cuda(ctx, cudaGetLastError(), "megakernel launch");
     }
     if (!use_graph || counting || !splat || ctx->profiling) return enqueue_wavefront(ctx, depth, paths, splat, counting);
-    // one graph per (depth, path capacity, sphere kernels, shade kernels); the batch itself lives in device memory
-    if (!ctx->graph || ctx->graph_depth != depth || ctx->graph_paths != ctx->path_cap ||
-        ctx->graph_spheres != ctx->batch_spheres || ctx->graph_kinds != ctx->batch_kinds) {
-        if (ctx->graph) {
-            cudaGraphExecDestroy(ctx->graph);
-            ctx->graph = nullptr;
+    // one graph per traversal variant, captured anew when the depth, the path capacity or the other
+    // kernels change; the batch itself lives in device memory
+    cgpu_ctx::Graph& G = ctx->graphs[ctx->batch_closest >= 2 ? 1 : 0];
+    if (!G.exec || G.depth != depth || G.paths != ctx->path_cap || G.spheres != ctx->batch_spheres ||
+        G.kinds != ctx->batch_kinds) {
+        if (G.exec) {
+            cudaGraphExecDestroy(G.exec);
+            G.exec = nullptr;
         }
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
@@ -1154,28 +1165,31 @@ cgpu_status run_batch(cgpu_ctx* ctx, int mode, int depth, uint32_t paths, bool s
         e = cudaStreamEndCapture(ctx->stream, &g);
         if (st != CGPU_OK) return st;
         if (e != cudaSuccess) return cg_cuda(ctx, e, "end capture");
-        e = cudaGraphInstantiate(&ctx->graph, g, 0);
+        e = cudaGraphInstantiate(&G.exec, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return cg_cuda(ctx, e, "graph instantiate");
-        ctx->graph_depth = depth;
-        ctx->graph_paths = ctx->path_cap;
-        ctx->graph_spheres = ctx->batch_spheres;
-        ctx->graph_kinds = ctx->batch_kinds;
-        ctx->graph_launches = ctx->stats.kernel_launches - before;
+        G.depth = depth;
+        G.paths = ctx->path_cap;
+        G.spheres = ctx->batch_spheres;
+        G.kinds = ctx->batch_kinds;
+        G.launches = ctx->stats.kernel_launches - before;
         ctx->stats.kernel_launches = before;
     }
-    ctx->stats.kernel_launches += ctx->graph_launches;
-    return cg_cuda(ctx, cudaGraphLaunch(ctx->graph, ctx->stream), "graph launch");
+    ctx->stats.kernel_launches += G.launches;
+    return cg_cuda(ctx, cudaGraphLaunch(G.exec, ctx->stream), "graph launch");
 }
 
 }  // namespace
 
-void cg_free_render_state(cgpu_ctx* ctx) {
-    if (ctx->graph) {
-        cudaGraphExecDestroy(ctx->graph);
-        ctx->graph = nullptr;
+void cg_drop_graphs(cgpu_ctx* ctx) {
+    for (cgpu_ctx::Graph& G : ctx->graphs) {
+        if (G.exec) cudaGraphExecDestroy(G.exec);
+        G = cgpu_ctx::Graph{};
     }
-    ctx->graph_depth = -1;
+}
+
+void cg_free_render_state(cgpu_ctx* ctx) {
+    cg_drop_graphs(ctx);
     if (ctx->wf_block) {
         cudaFree(ctx->wf_block);
         ctx->wf_block = nullptr;
@@ -1215,7 +1229,9 @@ cgpu_status cg_render_batches(cgpu_ctx* ctx, const cgpu_render_params* p) {
     }
     ctx->batch_spheres = false;
     ctx->batch_kinds = 0;
+    int records = 0;  // of the largest scene
     for (uint32_t i = 0; i < p->num_scenes; ++i) {
+        records = std::max(records, ctx->scenes[p->scenes[i]].d.num_tris);
         ctx->batch_spheres |= ctx->scenes[p->scenes[i]].has_spheres;
         ctx->batch_kinds |= ctx->scenes[p->scenes[i]].kinds;
     }
@@ -1236,6 +1252,13 @@ cgpu_status cg_render_batches(cgpu_ctx* ctx, const cgpu_render_params* p) {
             return cg_fail(ctx, CGPU_ERR_INVALID_ARGUMENT, "render: sample range overflows 32 bits");
         end[i] = p->first_sample + uint32_t(n);
     }
+    uint64_t asked = 0;
+    for (uint32_t i = 0; i < p->num_scenes; ++i) {
+        const SceneSlot& sl = ctx->scenes[p->scenes[i]];
+        asked += uint64_t(sl.width) * uint64_t(sl.height) * (end[i] - next[i]);
+    }
+    const bool persistent = records >= kLargeScene || (records >= kSmallScene && large_batch(ctx, asked));
+    choose_traversal(ctx, persistent, persistent);
     uint64_t total_paths = 0;
     for (;;) {
         uint32_t used = 0, pix = 0, nch = 0;
@@ -1307,6 +1330,9 @@ cgpu_status cg_render_paths_raw(cgpu_ctx* ctx, int scene, int mode, uint32_t fir
     if (st != CGPU_OK) return st;
     st = ensure_sort_buffers(ctx);
     if (st != CGPU_OK) return st;
+    const bool persistent =
+        sl.d.num_tris >= kLargeScene || (sl.d.num_tris >= kSmallScene && large_batch(ctx, uint64_t(count) * npix));
+    choose_traversal(ctx, persistent, persistent);
     float* d_out = nullptr;
     const uint32_t per = std::max<uint32_t>(1, ctx->path_cap / npix);
     cudaError_t e = cudaMalloc(&d_out, size_t(per) * npix * 3 * sizeof(float));
@@ -1439,17 +1465,17 @@ void enqueue_adjoint_pass(cgpu_ctx* ctx, const RenderArgs& a, int depth, uint32_
     const int bt = ctx->tuning.block_trace, bs = ctx->tuning.block_shade;
     const bool sph = ctx->batch_spheres;
     // the persistent passes when the tuning uses them (traversal 2 / 3), else the per-ray loops
-    const int trav = ctx->tuning.traversal;
+    const int trav = ctx->batch_closest, trav_any = ctx->batch_any;
     auto ext = trav >= 2 ? (sph ? k_wf_extend_pww<false, true> : k_wf_extend_pww<false, false>)
                          : (sph ? k_wf_extend<false, true> : k_wf_extend<false, false>);
-    auto shd = trav == 3 ? (sph ? k_wf_shadow_pww<false, true, true> : k_wf_shadow_pww<false, false, true>)
+    auto shd = trav_any == 3 ? (sph ? k_wf_shadow_pww<false, true, true> : k_wf_shadow_pww<false, false, true>)
                          : (sph ? k_wf_shadow<false, true, true> : k_wf_shadow<false, false, true>);
     auto mo = sph ? k_wf_mis_occl<false, true, true> : k_wf_mis_occl<false, false, true>;
     auto ties = sph ? k_wf_ties<false, true> : k_wf_ties<false, false>;
     void (*shade[kNumBsdfKinds])(RenderArgs, int) = {k_wf_shade<0, true>, k_wf_shade<1, true>, k_wf_shade<2, true>,
                                                      k_wf_shade<3, true>, k_wf_shade<4, true>};
     k_wf_generate<<<grid_for(ctx, k_wf_generate, kBlock, paths), kBlock, 0, s>>>(a);
-    const size_t ext_sm = stack_smem(ext, trav >= 2, true, bt), sh_sm = stack_smem(shd, trav == 3, false, bt);
+    const size_t ext_sm = stack_smem(ext, trav >= 2, true, bt), sh_sm = stack_smem(shd, trav_any == 3, false, bt);
     const int gext = grid_for(ctx, ext, bt, paths, ext_sm), gsh = grid_for(ctx, shd, bt, paths, sh_sm);
     const int gmo = grid_for(ctx, mo, bt, paths), gties = grid_for(ctx, ties, kTieBlock, paths);
     const int gv = grid_for(ctx, k_adj_vertex, kBlock, paths, shared_bytes);
@@ -1540,6 +1566,8 @@ cgpu_status cg_adjoint_wavefront(cgpu_ctx* ctx, int scene, uint32_t spp, uint64_
     a.adj.q_vtx[0] = ctx->adj.q_vtx[0];
     a.adj.q_vtx[1] = ctx->adj.q_vtx[1];
     ctx->stats = cgpu_render_stats{};
+    const bool persistent = sl.d.num_tris >= kSmallScene && large_batch(ctx, uint64_t(spp) * npix);
+    choose_traversal(ctx, persistent, persistent);
     const uint32_t per = std::max<uint32_t>(1, ctx->path_cap / npix);
     const int depth = sl.max_depth;
     for (uint32_t done = 0; done < spp;) {
@@ -1621,16 +1649,16 @@ cgpu_status noalloc_base(cgpu_ctx* ctx, char** out) {
 void enqueue_wavefront_serial(cgpu_ctx* ctx, const RenderArgs& a, int depth, uint32_t paths, uint32_t npix) {
     cudaStream_t s = ctx->stream;
     const int bt = ctx->tuning.block_trace, bs = ctx->tuning.block_shade;
-    const int trav = ctx->tuning.traversal;
+    const int trav = ctx->batch_closest, trav_any = ctx->batch_any;
     const bool sph = ctx->batch_spheres;
     auto ext = trav == 1   ? (sph ? k_wf_extend_dyn<false, true> : k_wf_extend_dyn<false, false>)
                : trav >= 2 ? (sph ? k_wf_extend_pww<false, true> : k_wf_extend_pww<false, false>)
                            : (sph ? k_wf_extend<false, true> : k_wf_extend<false, false>);
-    auto sh = trav == 1   ? (sph ? k_wf_shadow_dyn<false, true> : k_wf_shadow_dyn<false, false>)
-              : trav == 3 ? (sph ? k_wf_shadow_pww<false, true> : k_wf_shadow_pww<false, false>)
+    auto sh = trav_any == 1   ? (sph ? k_wf_shadow_dyn<false, true> : k_wf_shadow_dyn<false, false>)
+              : trav_any == 3 ? (sph ? k_wf_shadow_pww<false, true> : k_wf_shadow_pww<false, false>)
                           : (sph ? k_wf_shadow<false, true> : k_wf_shadow<false, false>);
     k_wf_generate<<<grid_for(ctx, k_wf_generate, kBlock, paths), kBlock, 0, s>>>(a);
-    const size_t ext_sm = stack_smem(ext, trav >= 2, true, bt), sh_sm = stack_smem(sh, trav == 3, false, bt);
+    const size_t ext_sm = stack_smem(ext, trav >= 2, true, bt), sh_sm = stack_smem(sh, trav_any == 3, false, bt);
     const int gext = grid_for(ctx, ext, bt, paths, ext_sm), gsh = grid_for(ctx, sh, bt, paths, sh_sm);
     const int gsd[kNumBsdfKinds] = {grid_for(ctx, k_wf_shade<0>, bs, paths), grid_for(ctx, k_wf_shade<1>, bs, paths),
                                     grid_for(ctx, k_wf_shade<2>, bs, paths), grid_for(ctx, k_wf_shade<3>, bs, paths),
@@ -1694,6 +1722,7 @@ extern "C" cgpu_status cgpu_render_noalloc(cgpu_ctx* ctx, int32_t scene, uint32_
     a.refill_closest = refill_lanes(ctx->tuning.refill_closest);
     a.refill_any = refill_lanes(ctx->tuning.refill_any);
     const uint32_t n = uint32_t(npix);
+    choose_traversal(ctx, false, sl.d.num_tris >= kSmallScene);
     const uint32_t per = kNoAllocMaxPaths / n;  // samples per batch
     const int depth = sl.max_depth;
     ctx->batch_spheres = sl.has_spheres;

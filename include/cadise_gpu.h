@@ -385,11 +385,14 @@ typedef struct cgpu_tuning {
     int32_t block_trace;   /* threads per block: extend, shadow and megakernel (32..1024, multiple of 32) */
     int32_t block_shade;   /* threads per block: shade-by-BSDF kernels */
     uint32_t max_paths;    /* paths in flight per wavefront batch; 0 = automatic (2^21, at least one frame) */
-    int32_t traversal;     /* 0: one ray per thread per grid-stride step; 1: persistent warps that hand a
-                              finished lane the next ray at once; 2: persistent while-while closest-hit
-                              pass that refills a warp's finished lanes once fewer than refill_closest
-                              of its lanes still trace; 3: 2 plus the same persistent while-while form
-                              for the any-hit pass (refill_any) */
+    int32_t traversal;     /* 0: the library's choice by scene and batch size (default): 3 where its passes
+                              are the faster ones (scenes of 16,384 triangles, or of 512 in batches of 2^19
+                              paths), else one ray per thread per grid-stride step; 1: persistent warps that hand
+                              a finished lane the next ray at once; 2: persistent closest-hit pass that
+                              votes between node and triangle steps and refills a warp's finished lanes
+                              once fewer than refill_closest of its lanes still trace, any-hit with one
+                              ray per thread; 3: 2 plus the same persistent form for the any-hit pass
+                              (refill_any) */
     int32_t reorder;       /* 1, 2, 3: before each closest-hit pass after the first, sort its rays by
                               direction octant and origin (Morton order of 9, 7 or 4 bits per axis in the
                               scene bounds; 4, 3 or 2 radix passes), so that a warp traces neighbouring
