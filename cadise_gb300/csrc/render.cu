@@ -1013,11 +1013,13 @@ void collect_profile(cgpu_ctx* ctx) {
 }
 
 // The traversal variants of the current render's passes: the tuning's, or where
-// it leaves them open the persistent ones if the caller may use them (below).
+// it leaves them open the persistent ones as the caller asks.  Counting renders
+// then keep one ray per thread, whose node visits do not depend on which rays
+// happen to share a warp.
 void choose_traversal(cgpu_ctx* ctx, bool closest, bool any) {
     const int t = ctx->tuning.traversal;
-    ctx->batch_closest = t == 0 && closest ? 3 : t;
-    ctx->batch_any = t == 0 && any ? 3 : t;
+    ctx->batch_closest = t == 0 && closest && !ctx->counting ? 3 : t;
+    ctx->batch_any = t == 0 && any && !ctx->counting ? 3 : t;
 }
 bool large_batch(const cgpu_ctx* ctx, uint64_t paths) { return std::min<uint64_t>(paths, ctx->path_cap) >= kLargeBatch; }
 
