@@ -150,8 +150,9 @@ CG_D void pray_prep(PRay<SPH>& r, float3 d) {
 
 // One pass over the `n` rays of a queue.  fetch(k, &o, &d, &tmin, &tmax, &scene)
 // loads entry k and returns the caller's id of the ray; finish(done, id, t,
-// slot, kind, tie) is called by the whole warp with the lanes whose ray is done
-// (slot < 0: a miss; kind: the record's shade queue; tie: two candidates within the tie window);
+// slot, kind, other) is called by the whole warp with the lanes whose ray is done
+// (slot < 0: a miss; kind: the record's shade queue; other: the record that met
+// the ray within the tie window of slot, -1 none, -2 more than one);
 // exhausted(id): the ray ran out of its visit budget.
 // GENERAL (ray queries): every ray has its own tmin, and closest-hit rays cull
 // nodes by the tie window's far end, so that every primitive within the window
@@ -169,7 +170,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
     float tie_abs = 0.0f;
     float tcur = 0.0f, ray_tmin = 0.0f;
     int hslot = -1;
-    bool tie = false;
+    int other = -1;      // the record within the tie window of hslot: -1 none, -2 more than one
     int left = 0;        // node and leaf visits left, negative once the budget is exceeded
     int cur = -1;        // next entry: an inner node (>= 0), a leaf (< -1), -1 none
     int leaf = -1;       // postponed leaf, -1 none
@@ -206,7 +207,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                 left = int(min(S->visit_budget, 0x7FFFFFFFu));
                 pray_prep(r, d);
                 hslot = -1;
-                tie = false;
+                other = -1;
                 cur = 0;
                 leaf = -1;
                 stack.clear();
@@ -356,8 +357,14 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                         cur = leaf = -1;
                         stack.clear();
                     } else {
-                        if (hslot >= 0 && t * kTieSlack + tie_abs >= tcur) tie = true;
-                        if (hslot < 0 ? t <= tcur : (t < tcur || (t == tcur && int(slot) < (hslot & kSlotMask)))) {
+                        const bool first = hslot < 0;
+                        const int held = hslot & kSlotMask;
+                        const bool nearer = first ? t <= tcur : (t < tcur || (t == tcur && int(slot) < held));
+                        // a hit nearer by more than the window clears what the held one was tied with
+                        const bool tied = !first && t * kTieSlack + tie_abs >= tcur;
+                        if (tied) other = other == -1 ? (nearer ? held : int(slot)) : -2;
+                        else if (nearer) other = -1;
+                        if (nearer) {
                             // the record's shade queue rides above its 28 slot bits
                             hslot = int(slot | (__float_as_uint(c.w) >> kRecQueueShift << 28));
                             tcur = t;
@@ -375,7 +382,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
         const bool over = left < 0 || (left == 0 && cur >= 0);
         const bool done = p >= 0 && (over || (cur == -1 && leaf == -1 && stack.sp == stack.base));
         if (done && over) exhausted(p);
-        finish(done, p, tcur, hslot < 0 ? -1 : hslot & kSlotMask, hslot >> 28, tie);
+        finish(done, p, tcur, hslot < 0 ? -1 : hslot & kSlotMask, hslot >> 28, other);
         if (done) {
             p = -1;
             cur = leaf = -1;

@@ -351,10 +351,12 @@ __global__ void __maxnreg__(kPersistRegs) k_wf_extend_pww(RenderArgs a, int b) {
             if (COUNT) ++nclosest;
             return p;
         },
-        [&](bool done, int p, float t, int slot, int kind, bool tie) {
+        [&](bool done, int p, float t, int slot, int kind, int other) {
             if (!done) return;
-            if (tie) w.q_tie[atomicAdd(cnt + 12, 1)] = p;
-            else extend_finish(w, a.scenes[__ldcs(&w.meta[p].x)], cnt + 3, p, t, slot, kind);
+            if (other != -1) {
+                w.hit[p] = make_float4(t, __int_as_float(slot), __int_as_float(other), 0.0f);
+                w.q_tie[atomicAdd(cnt + 12, 1)] = p;
+            } else extend_finish(w, a.scenes[__ldcs(&w.meta[p].x)], cnt + 3, p, t, slot, kind);
         },
         [&](int p) {
             uint32_t* st = a.scenes[w.meta[p].x].status;
@@ -366,12 +368,38 @@ __global__ void __maxnreg__(kPersistRegs) k_wf_extend_pww(RenderArgs a, int b) {
 
 constexpr int kTieBlock = 64;
 
+// The hit of a closest-hit ray that the persistent pass left with `held` and
+// another record within the tie window (`other`; -2: several, the ray is traced
+// again from scratch): held or other by closer_hit's rules, other's distance
+// worked out again by the same test.
+template <bool COUNT, bool SPH>
+CG_D HitD tie_hit(const SceneD& S, const RayPre& r, HitD held, int other, TraceCounters* cnt) {
+    if (other < 0) {
+        if (!traverse<false, COUNT, SPH>(S, r, &held, cnt)) held.slot = -1;
+        return held;
+    }
+    const float4* tp = reinterpret_cast<const float4*>(S.tris + other);
+    const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
+    float t, u, v;
+    const float bound = tie_hi(S, tie_hi(S, held.t));
+    const bool sphere = SPH && (__float_as_uint(c.w) & 3u) == kRecSphere;
+    if ((sphere ? sphere_test(r, f3(a), b.x, bound, &t) : tri_test(r, f3(a), f3(b), f3(c), bound, &t, &u, &v)) &&
+        closer_hit(S, r, t, __float_as_int(a.w), other, held.t, held.slot)) {
+        held.t = t;
+        held.slot = other;
+    }
+    return held;
+}
+
 // Closest-hit rays the persistent pass left to this kernel (q_tie): two
 // primitives within the tie window of each other, which tie_prefers orders
-// by the reference's own test and tie order.  Traced again with the per-ray
-// traversal (closer_hit / tie_prefers, wide culling), then finished as the
-// persistent pass finishes its other rays.  It runs beside the any-hit pass
-// (on the other stream), and its grid strides over however few rays it got.
+// by the reference's own test and tie order.  Of two the pass has both records
+// and only the comparison is left; of more the ray is traced again with the
+// per-ray traversal (closer_hit / tie_prefers, wide culling).  Then it is
+// finished as the persistent pass finishes its other rays.  Bound by latency:
+// few rays, and a launch that traced each of them again lasted 120 to 150 us
+// whatever their number.  It runs beside the any-hit pass (on the other
+// stream), and its grid strides over however few rays it got.
 template <bool COUNT, bool SPH>
 __global__ void k_wf_ties(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
@@ -384,8 +412,11 @@ __global__ void k_wf_ties(RenderArgs a, int b) {
         const int p = w.q_tie[i];
         const SceneD& S = a.scenes[w.meta[p].x];
         const RayPre r = ray_prep(f3(w.ray_o[p]), f3(w.ray_d[p]), kRayEps, kFloatMax);
+        const float4 h4 = w.hit[p];
         HitD hit;
-        if (!traverse<false, COUNT, SPH>(S, r, &hit, &tc)) hit.slot = -1;
+        hit.t = h4.x;
+        hit.slot = __float_as_int(h4.y);
+        hit = tie_hit<COUNT, SPH>(S, r, hit, __float_as_int(h4.z), &tc);
         extend_finish(w, S, cnt + 3, p, hit.t, hit.slot, kind_of_slot(S, hit.slot));
     }
     count_flush<COUNT>(a.counters, tc, TraceCounters{0, 0}, 0, 0);
@@ -414,7 +445,7 @@ __global__ void __maxnreg__(kPersistRegs) k_wf_shadow_pww(RenderArgs a, int b) {
             if (COUNT) ++nany;
             return p;
         },
-        [&](bool done, int p, float, int slot, int, bool) {
+        [&](bool done, int p, float, int slot, int, int) {
             if (done) shadow_finish<ADJ>(w, p, slot >= 0);
         },
         [&](int p) {
@@ -804,10 +835,10 @@ __global__ void k_trace(const SceneD* scenes, int scene, const cgpu_ray* rays, u
 }
 
 // Large batches of queries: the persistent pass, then (closest hit) one thread
-// per ray for the answer.  k_query_closest leaves the traversal's distance in
-// hits[i].t and its record slot in hits[i].primitive (-1: a miss), ~slot - 1
-// for a ray that met two candidates within the tie window, which
-// k_query_resolve traces again with the tie rule from the hit it holds.
+// per ray for the answer.  k_query leaves the traversal's distance in hits[i].t,
+// its record slot in hits[i].primitive (-1: a miss) and the record within its
+// tie window in hits[i].u, as the pass reports it; k_query_resolve compares the
+// two (tie_hit).
 CG_D void load_query(const cgpu_ray& r, float3* o, float3* d, float* tmin, float* tmax) {
     *o = mk(r.org[0], r.org[1], r.org[2]);
     // the direction is normalised again, as the reference's Ray constructor does (ray.cpp:19-30)
@@ -827,13 +858,14 @@ __global__ void __maxnreg__(kPersistRegs) k_query(const SceneD* scenes, int scen
             *s = scene;
             return k;
         },
-        [&](bool done, int k, float t, int slot, int, bool tie) {
+        [&](bool done, int k, float t, int slot, int, int other) {
             if (!done) return;
             if (ANY) {
                 occ[k] = slot >= 0 ? 1 : 0;
             } else {
                 hits[k].t = t;
-                hits[k].primitive = tie ? -slot - 2 : slot;
+                hits[k].primitive = slot;
+                hits[k].u = __int_as_float(other);
             }
         },
         [&](int) {
@@ -853,10 +885,10 @@ __global__ void k_query_resolve(const SceneD* scenes, int scene, const cgpu_ray*
         h.t = hits[i].t;
         h.slot = hits[i].primitive;
         h.u = h.v = 0.0f;
-        if (h.slot < -1) {
-            h.slot = -h.slot - 2;
+        const int other = __float_as_int(hits[i].u);
+        if (h.slot >= 0 && other != -1) {
             TraceCounters tc{0, 0};
-            traverse<false, false>(S, ray_prep(o, d, tmin, tmax), &h, &tc, true);
+            h = tie_hit<false, true>(S, ray_prep(o, d, tmin, tmax), h, other, &tc);
         }
         hits[i] = query_answer(S, o, d, h);
     }

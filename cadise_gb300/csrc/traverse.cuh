@@ -437,14 +437,13 @@ CG_D bool visit_leaf(const SceneD& S, const RayPre& r, uint32_t e, float& tcur, 
 // One ray per thread, one node or one leaf per loop iteration: the
 // megakernel's traversal (its threads are at different bounces anyway) and
 // every any-hit query (the first hit ends the walk, so there is nothing to
-// gain from holding leaves back).  `held`: *hit is a hit the ray is known to
-// have; a closest-hit walk then starts from its distance.
+// gain from holding leaves back).
 template <bool ANY, bool COUNT, bool SPH = true>
-CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* cnt, bool held = false) {
+CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* cnt) {
     LocalStack stack;
     int sp = 0;
-    float tcur = held ? hit->t : r.tmax;
-    int hslot = held ? hit->slot : -1;
+    float tcur = r.tmax;
+    int hslot = -1;
     float hu = 0.0f, hv = 0.0f;
     uint32_t cur = 0;  // root first (always an inner node)
     uint32_t left = S.visit_budget;
