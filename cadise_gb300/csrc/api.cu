@@ -208,6 +208,7 @@ void cgpu_destroy(cgpu_ctx* ctx) {
     if (ctx->d_chunks) cudaFree(ctx->d_chunks);
     if (ctx->d_header) cudaFree(ctx->d_header);
     if (ctx->query_block) cudaFree(ctx->query_block);
+    if (ctx->grad_block) cudaFree(ctx->grad_block);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->h_chunks) cudaFreeHost(ctx->h_chunks);
     if (ctx->h_header) cudaFreeHost(ctx->h_header);

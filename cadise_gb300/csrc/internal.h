@@ -272,6 +272,9 @@ struct cgpu_ctx {
     uint32_t adj_cap = 0;
     cg::AdjBufs adj{};
     void* adj_block = nullptr;
+    // gradient and image buffers of the adjoint calls (adjoint.cu)
+    void* grad_block = nullptr;
+    size_t grad_cap = 0;
     int adjoint_schedule = CGPU_MODE_WAVEFRONT;
     int bvh_builder = CGPU_BVH_BUILDER_AUTO;
     int tie_order = CGPU_TIE_ORDER_REFERENCE;
