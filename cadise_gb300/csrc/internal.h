@@ -22,7 +22,7 @@ struct Chunk {
     uint32_t sample0;
     uint32_t nsamples;
     uint32_t pix_begin;  // prefix over chunks of npix (film splat index space)
-    uint32_t pad;
+    uint32_t pixel0;     // first pixel of the scene in this chunk (0 but for the adjoint's frames in parts)
 };
 constexpr int kMaxChunks = 256;
 
@@ -44,7 +44,7 @@ struct FilmD {
 //   k = 0 continuation rays to extend, 1 unused, 2 shadow rays,
 //   3 + kind: hits waiting for the shade kernel of that BSDF kind,
 //   8 / 9: rays handed out so far by the persistent extend / shadow kernels,
-//   10: adjoint vertices of bounce b - 1 (the wavefront adjoint's gradient kernel),
+//   10: unused,
 //   11: MIS rays whose direction meets the sampled light's primitive (or that
 //       sampled the environment), left for the MIS occlusion pass,
 //   12: closest-hit rays of the persistent pass left for k_wf_ties (q_tie).
@@ -136,17 +136,13 @@ inline size_t noalloc_layout(char* base, NoAllocView* v) {
     return off + wf_layout(base ? base + off : nullptr, kNoAllocMaxPaths, kNoAllocMaxDepth + 2, &v->wf);
 }
 
-// Wavefront adjoint (path replay in wavefront form): per path the radiance
-// of the whole path from a first wavefront pass (Ltot), the radiance of the
-// vertices replayed so far (acc), and what one vertex leaves for the gradient
-// kernel that runs once its shadow and MIS rays are traced: st_a = textured
-// albedo and texel index, st_b = d ln f / d roughness towards the shadow,
-// MIS and continuation directions + material | flags, st_c = the shadow
-// contribution without the light's radiance + the light; mis_B / mis_X = the
-// MIS half and its radiance derivative (with the light) once resolved.
+// Wavefront adjoint (path replay in wavefront form): per path the radiance of
+// the whole path from the forward pass (Ltot) and of the vertices replayed so
+// far (acc); per path and bounce what the forward pass's rays found, so that
+// the replay traces none: the hit, the shade queues, and a byte each for the
+// shadow ray and the MIS ray (1: nothing in the way).
 struct AdjBufs {
-    float4 *Ltot, *acc, *st_a, *st_b, *st_c, *mis_B, *mis_X;
-    int* q_vtx[2];          // paths with a vertex at bounce b, ping-pong on b
+    float4 *Ltot, *acc;
     const float* dLdI;      // d loss / d pixel, 3 per pixel
     double* g_tex;
     const int* tex_offset;  // per texture: first float of its block in g_tex
@@ -155,20 +151,39 @@ struct AdjBufs {
     int nmat, nlight;
     float inv_spp;
 };
-// st_b.w bits above the 16-bit material index
-constexpr uint32_t kAdjShadow = 1u << 16, kAdjMis = 1u << 17, kAdjCont = 1u << 18, kAdjTexel = 1u << 19,
-                   kAdjGgx = 1u << 20;
 
-inline size_t adj_layout(char* base, size_t cap, AdjBufs* a) {
+// The records of one batch: arrays of `depth` rows, one entry per path in each.
+struct AdjRecords {
+    size_t stride = 0;  // entries a row
+    int depth = 0;
+    float4* hit = nullptr;
+    int* q_mat[kNumBsdfKinds] = {};
+    uint8_t *shadow = nullptr, *mis = nullptr;
+};
+
+// Bytes of records a path takes.
+inline size_t adj_record_bytes(uint32_t kinds, int depth) {
+    size_t row = sizeof(float4) + 2;
+    for (int k = 0; k < kNumBsdfKinds; ++k) row += (kinds >> k & 1u) * sizeof(int);
+    return row * size_t(depth > 0 ? depth : 1);
+}
+
+inline size_t adj_layout(char* base, size_t paths, uint32_t kinds, int depth, AdjBufs* a, AdjRecords* r) {
     size_t off = 0;
     auto take = [&](size_t bytes) {
-        char* r = base ? base + off : nullptr;
+        char* q = base ? base + off : nullptr;
         off += (bytes + 255) & ~size_t(255);
-        return r;
+        return q;
     };
-    float4** f4s[] = {&a->Ltot, &a->acc, &a->st_a, &a->st_b, &a->st_c, &a->mis_B, &a->mis_X};
-    for (float4** f : f4s) *f = reinterpret_cast<float4*>(take(cap * sizeof(float4)));
-    for (int k = 0; k < 2; ++k) a->q_vtx[k] = reinterpret_cast<int*>(take(cap * sizeof(int)));
+    r->stride = paths;
+    r->depth = depth > 0 ? depth : 1;
+    const size_t n = paths * size_t(r->depth);
+    a->Ltot = reinterpret_cast<float4*>(take(paths * sizeof(float4)));
+    a->acc = reinterpret_cast<float4*>(take(paths * sizeof(float4)));
+    r->hit = reinterpret_cast<float4*>(take(n * sizeof(float4)));
+    for (int k = 0; k < kNumBsdfKinds; ++k) r->q_mat[k] = kinds >> k & 1u ? reinterpret_cast<int*>(take(n * sizeof(int))) : nullptr;
+    r->shadow = reinterpret_cast<uint8_t*>(take(n));
+    r->mis = reinterpret_cast<uint8_t*>(take(n));
     return off;
 }
 
@@ -180,6 +195,9 @@ struct RenderArgs {
     WfBuffers wf;
     unsigned long long* counters;  // closest rays, any rays, nodes, tris, paths
     AdjBufs adj;      // wavefront adjoint only
+    // wavefront adjoint: where the passes record (forward) or find (replay) the
+    // outcome of one bounce's shadow and MIS rays; null in other renders
+    uint8_t *rec_shadow, *rec_mis;
     // reordered closest-hit queue (tuning.reorder): paths
     const uint32_t* sorted;
     // persistent traversal passes: a warp refills its finished lanes once
@@ -264,13 +282,12 @@ struct cgpu_ctx {
     uint32_t path_cap = 0;
     cg::WfBuffers wf{};
     void* wf_block = nullptr;
-    // wavefront adjoint state (allocated by the first wavefront adjoint)
+    // wavefront adjoint state (Ltot, acc, records), kept between calls
     // ray reordering buffers (allocated while tuning.reorder is on)
     uint32_t sort_cap = 0;
     cg::SortBufs sort{};
     void* sort_block = nullptr;
-    uint32_t adj_cap = 0;
-    cg::AdjBufs adj{};
+    size_t adj_bytes = 0;
     void* adj_block = nullptr;
     // gradient and image buffers of the adjoint calls (adjoint.cu)
     void* grad_block = nullptr;

@@ -27,7 +27,7 @@ CG_D PathId path_id(const Chunk* chunks, int nchunks, uint32_t p) {
     PathId id;
     id.scene = c.scene;
     id.sample = c.sample0 + local / c.npix;
-    id.pixel = local % c.npix;
+    id.pixel = c.pixel0 + local % c.npix;
     id.width = c.width;
     return id;
 }

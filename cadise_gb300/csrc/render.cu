@@ -127,11 +127,23 @@ CG_D int kind_of_slot(const SceneD& S, int slot) {
     return slot < 0 ? -1 : int(__float_as_uint(ldg4(reinterpret_cast<const float4*>(S.tris + slot) + 2).w) >> kRecQueueShift);
 }
 
+// What an unoccluded MIS ray from o along d adds that meets its light at mh
+// (mis_light_hit; mh.y: record, -1 the environment).  X (optional): its
+// derivative by the light's radiance.
+CG_D float3 mis_add(const SceneD& S, float3 o, float3 d, float4 mh, float3 T, float3 factor, float pdf, float3* X) {
+    HitD hit;
+    hit.t = mh.x;
+    hit.slot = __float_as_int(mh.y);
+    hit.u = mh.z;
+    hit.v = mh.w;
+    if (hit.slot < 0) return mis_resolve_env(S, d, T, factor, pdf);
+    return mis_resolve(S, surface_at(S, o, d, hit), o, T, factor, pdf, X);
+}
+
 // MIS rays that meet their light (mis_light_hit): unless a primitive comes
 // before the light's hit, the BSDF-sampling half of the NEE estimate, added to
-// L (ADJ: stored with its radiance derivative for the adjoint's gradient
-// kernel).
-template <bool COUNT, bool SPH, bool ADJ = false>
+// L (and recorded for the adjoint's replay).
+template <bool COUNT, bool SPH>
 __global__ void k_wf_mis_occl(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
     const int n = w.cnt[b * kCntStride + 11];
@@ -146,27 +158,11 @@ __global__ void k_wf_mis_occl(RenderArgs a, int b) {
         const int slot = __float_as_int(mh.y);
         const int prim_l = slot >= 0 ? __float_as_int(ldg4(reinterpret_cast<const float4*>(S.tris + slot)).w) : 0x7FFFFFFF;
         if (COUNT) ++nany;
-        if (occluded_before<COUNT, SPH>(S, r, mh.x, prim_l, slot, &tc)) continue;
+        const bool occluded = occluded_before<COUNT, SPH>(S, r, mh.x, prim_l, slot, &tc);
+        if (a.rec_mis) a.rec_mis[p] = occluded ? 0 : 1;
+        if (occluded) continue;
         const float4 mb = w.mis_b[p], ma = w.mis_a[p];
-        float3 add, X = splat3(0.0f);
-        int xlight = -1;
-        if (slot >= 0) {
-            HitD hit;
-            hit.t = mh.x;
-            hit.slot = slot;
-            hit.u = mh.z;
-            hit.v = mh.w;
-            const SurfaceD hs = surface_at(S, r.o, r.d, hit);
-            add = mis_resolve(S, hs, r.o, f3(mb), f3(ma), ma.w, ADJ ? &X : nullptr);
-            xlight = __float_as_int(mb.w);
-        } else {
-            add = mis_resolve_env(S, r.d, f3(mb), f3(ma), ma.w);
-        }
-        if (ADJ) {
-            a.adj.mis_B[p] = make_float4(add.x, add.y, add.z, 1.0f);
-            a.adj.mis_X[p] = make_float4(X.x, X.y, X.z, __int_as_float(xlight));
-            continue;
-        }
+        const float3 add = mis_add(S, r.o, r.d, mh, f3(mb), f3(ma), ma.w, nullptr);
         float4 L = w.L[p];
         L.x += add.x;
         L.y += add.y;
@@ -176,15 +172,11 @@ __global__ void k_wf_mis_occl(RenderArgs a, int b) {
     count_flush<COUNT>(a.counters, TraceCounters{0, 0}, tc, 0, nany);
 }
 
-// ADJ: marks an unoccluded shadow ray in sh_c.w for the adjoint's gradient kernel.
-template <bool ADJ = false>
-CG_D void shadow_finish(const WfBuffers& w, int p, bool occluded) {
+// After the trace of path p's shadow ray (rec: recorded for the adjoint's replay).
+CG_D void shadow_finish(const WfBuffers& w, uint8_t* rec, int p, bool occluded) {
+    if (rec) rec[p] = occluded ? 0 : 1;
     if (occluded) return;
     const float4 c = w.sh_c[p];
-    if (ADJ) {
-        w.sh_c[p] = make_float4(c.x, c.y, c.z, 1.0f);
-        return;
-    }
     float4 Ls = w.Ls[p];
     Ls.x += c.x;
     Ls.y += c.y;
@@ -246,7 +238,7 @@ __global__ void k_wf_extend(RenderArgs a, int b) {
     count_flush<COUNT>(a.counters, tc, TraceCounters{0, 0}, nclosest, 0);
 }
 
-template <bool COUNT, bool SPH, bool ADJ = false>
+template <bool COUNT, bool SPH>
 __global__ void k_wf_shadow(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
     const int n = w.cnt[b * kCntStride + 2];
@@ -260,7 +252,7 @@ __global__ void k_wf_shadow(RenderArgs a, int b) {
         const RayPre r = ray_prep(f3(w.ray_o[p]), f3(sd), kRayEps, sd.w);
         HitD hit;
         if (COUNT) ++nany;
-        shadow_finish<ADJ>(w, p, traverse<true, COUNT, SPH>(S, r, &hit, &tc));
+        shadow_finish(w, a.rec_shadow, p, traverse<true, COUNT, SPH>(S, r, &hit, &tc));
     }
     count_flush<COUNT>(a.counters, TraceCounters{0, 0}, tc, 0, nany);
 }
@@ -424,8 +416,7 @@ __global__ void k_wf_ties(RenderArgs a, int b) {
 }
 
 // Persistent any-hit pass over the shadow rays; a ray ends at its first hit.
-
-template <bool COUNT, bool SPH, bool ADJ = false>
+template <bool COUNT, bool SPH>
 __global__ void __maxnreg__(kPersistRegs) k_wf_shadow_pww(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
     int* cnt = w.cnt + b * kCntStride;
@@ -446,7 +437,7 @@ __global__ void __maxnreg__(kPersistRegs) k_wf_shadow_pww(RenderArgs a, int b) {
             return p;
         },
         [&](bool done, int p, float, int slot, int, int) {
-            if (done) shadow_finish<ADJ>(w, p, slot >= 0);
+            if (done) shadow_finish(w, a.rec_shadow, p, slot >= 0);
         },
         [&](int p) {
             uint32_t* st = a.scenes[w.meta[p].x].status;
@@ -488,7 +479,7 @@ __global__ void k_wf_shadow_dyn(RenderArgs a, int b) {
             const SceneD& S = a.scenes[w.meta[p].x];
             for (int s = 0; s < kStepsPerFetch && !st.done; ++s) trav_step<true, COUNT, SPH>(S, r, st, &tc);
             if (st.done) {
-                shadow_finish(w, p, st.hslot >= 0);
+                shadow_finish(w, a.rec_shadow, p, st.hslot >= 0);
                 i = -1;
             }
         }
@@ -513,129 +504,33 @@ CG_D void adj_shared_flush(double* sh, const AdjBufs& A) {
 CG_D void adj_add(double* sh, int i, double v) {
     if (v != 0.0) atomicAdd(sh + i, v);
 }
+CG_D void adj_radiance(double* sh, const AdjBufs& A, int light, float3 g) {
+    adj_add(sh + A.nmat, 3 * light + 0, g.x);
+    adj_add(sh + A.nmat, 3 * light + 1, g.y);
+    adj_add(sh + A.nmat, 3 * light + 2, g.z);
+}
 CG_D float3 adj_delta(const AdjBufs& A, uint32_t pixel) {
     return mk(A.dLdI[3 * pixel] * A.inv_spp, A.dLdI[3 * pixel + 1] * A.inv_spp, A.dLdI[3 * pixel + 2] * A.inv_spp);
 }
 
-// The adjoint's part of shading vertex b of path p (the replay of adjoint.cuh,
-// split at the point where the vertex's shadow and MIS rays are traced): the
-// emission term's radiance gradient now, the rest kept for k_adj_vertex.
-// Returns whether the path carries gradient (finite total, nonzero weight).
-CG_D bool adj_vertex_begin(const RenderArgs& a, double* sh, const SceneD& S, const SurfaceD& si, const VertexPlan& pl,
-                           float4 tw, int p, uint32_t pixel) {
-    const AdjBufs& A = a.adj;
-    const float3 delta = adj_delta(A, pixel);
-    if (!finite3(f3(A.Ltot[p])) || is_zero(delta)) return false;
-    const bool ce = (__float_as_int(tw.w) & 1) != 0;
-    if (si.light >= 0 && si.light < A.nlight && ce && can_emit(S.lights[si.light], si.wi, si.Ns)) {
-        const float3 gx = delta * f3(tw);
-        adj_add(sh + A.nmat, 3 * si.light + 0, gx.x);
-        adj_add(sh + A.nmat, 3 * si.light + 1, gx.y);
-        adj_add(sh + A.nmat, 3 * si.light + 2, gx.z);
-    }
-    const float4 acc = A.acc[p];
-    A.acc[p] = make_float4(acc.x + pl.emit.x, acc.y + pl.emit.y, acc.z + pl.emit.z, 0.0f);
-    const MaterialD& m = S.materials[si.material];
-    uint32_t bits = uint32_t(si.material) | (pl.shadow ? kAdjShadow : 0u) | (pl.mis ? kAdjMis : 0u) |
-                    (pl.cont ? kAdjCont : 0u);
-    if (m.type == BSDF_LAMBERTIAN && m.albedo_tex >= 0) {
-        const TextureD& tex = S.textures[m.albedo_tex];
-        const float3 alb = texture_rgb(tex, si.uvw);
-        A.st_a[p] = make_float4(alb.x, alb.y, alb.z, __int_as_float(3 * texel_index(tex, si.uvw)));
-        bits |= kAdjTexel;
-    }
-    float gs = 0.0f, gb = 0.0f, gc = 0.0f;
-    if (m.type == BSDF_CONDUCTOR || m.type == BSDF_DIELECTRIC_GGX) {
-        if (pl.shadow) gs = dlogf_droughness(m, si.wi, pl.sdir, si.Ns);
-        if (pl.mis) gb = dlogf_droughness(m, si.wi, pl.mdir, si.Ns);
-        if (pl.cont) gc = dlogf_droughness(m, si.wi, pl.cdir, si.Ns);
-        bits |= kAdjGgx;
-    }
-    A.st_b[p] = make_float4(gs, gb, gc, __uint_as_float(bits));
-    if (pl.shadow) A.st_c[p] = make_float4(pl.sx.x, pl.sx.y, pl.sx.z, __int_as_float(pl.slight));
-    if (pl.mis) A.mis_B[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    return true;
-}
-
-// Vertices of bounce b, once their shadow (bounce b + 1 shadow pass) and MIS
-// (bounce b + 1 extend pass) rays are traced: A, B and the radiance of the
-// vertices after this one (R = Ltot - acc - A - B) give the texel, roughness
-// and radiance terms of adjoint.cuh.
-__global__ void k_adj_vertex(RenderArgs a, int b) {
-    extern __shared__ double sh[];
-    const WfBuffers& w = a.wf;
-    const AdjBufs& A = a.adj;
-    adj_shared_zero(sh, A);
-    const int n = w.cnt[(b + 1) * kCntStride + 10];
-    const int* q = A.q_vtx[b & 1];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int p = q[i];
-        const uint4 meta = w.meta[p];
-        const SceneD& S = a.scenes[meta.x];
-        const float3 delta = adj_delta(A, meta.y);
-        const float4 sb = A.st_b[p];
-        const uint32_t bits = __float_as_uint(sb.w);
-        const int mat = int(bits & 0xFFFFu);
-        float3 Av = splat3(0.0f), Bv = splat3(0.0f);
-        if (bits & kAdjShadow) {
-            const float4 c = w.sh_c[p];
-            if (c.w != 0.0f) {
-                Av = f3(c);
-                const float4 sc = A.st_c[p];
-                const int slight = __float_as_int(sc.w);
-                if (slight < A.nlight) {
-                    const float3 gx = delta * f3(sc);
-                    adj_add(sh + A.nmat, 3 * slight + 0, gx.x);
-                    adj_add(sh + A.nmat, 3 * slight + 1, gx.y);
-                    adj_add(sh + A.nmat, 3 * slight + 2, gx.z);
-                }
-            }
-        }
-        if (bits & kAdjMis) {
-            const float4 mb = A.mis_B[p];
-            if (mb.w != 0.0f) {
-                Bv = f3(mb);
-                const float4 mx = A.mis_X[p];
-                const int xl = __float_as_int(mx.w);
-                if (xl >= 0 && xl < A.nlight) {
-                    const float3 gx = delta * f3(mx);
-                    adj_add(sh + A.nmat, 3 * xl + 0, gx.x);
-                    adj_add(sh + A.nmat, 3 * xl + 1, gx.y);
-                    adj_add(sh + A.nmat, 3 * xl + 2, gx.z);
-                }
-            }
-        }
-        const float3 acc = f3(A.acc[p]);
-        const float3 after = f3(A.Ltot[p]) - acc - Av - Bv;
-        if (bits & kAdjTexel) {
-            const float4 sa = A.st_a[p];
-            const float3 num = delta * (Av + Bv + after);
-            double* g = A.g_tex + A.tex_offset[S.materials[mat].albedo_tex] + __float_as_int(sa.w);
-            if (sa.x > 0.0f && num.x != 0.0f) atomicAdd(g + 0, double(num.x / sa.x));
-            if (sa.y > 0.0f && num.y != 0.0f) atomicAdd(g + 1, double(num.y / sa.y));
-            if (sa.z > 0.0f && num.z != 0.0f) atomicAdd(g + 2, double(num.z / sa.z));
-        }
-        if (bits & kAdjGgx) {
-            float gr = 0.0f;
-            if (!is_zero(Av)) gr += dot(delta, Av) * sb.x;
-            if (!is_zero(Bv)) gr += dot(delta, Bv) * sb.y;
-            if (bits & kAdjCont) gr += dot(delta, after) * sb.z;
-            adj_add(sh, mat, double(gr));
-        }
-        const float3 nacc = acc + (Av + Bv);
-        A.acc[p] = make_float4(nacc.x, nacc.y, nacc.z, 0.0f);
-    }
-    adj_shared_flush(sh, A);
-}
-
-// Between the two wavefront passes of the adjoint: every path's total
-// radiance from the first, and a zero replay accumulator for the second.
-__global__ void k_adj_ltot(RenderArgs a) {
+// Before the replay: every path's total radiance from the forward pass, a zero
+// accumulator, and the path's state back at the camera (its shading draws the
+// same numbers again).
+__global__ void k_adj_begin(RenderArgs a) {
     const BatchHeader h = *a.header;
+    const WfBuffers& w = a.wf;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < h.total_paths; p += gridDim.x * blockDim.x) {
-        const float3 v = path_sample(f3(a.wf.L[p]), f3(a.wf.Le[p]), f3(a.wf.Ls[p]));
+        const float3 v = path_sample(f3(w.L[p]), f3(w.Le[p]), f3(w.Ls[p]));
         a.adj.Ltot[p] = make_float4(v.x, v.y, v.z, 0.0f);
         a.adj.acc[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const PathId id = path_id(a.chunks, int(h.num_chunks), p);
+        Rng rng;
+        float3 o, d;
+        primary_ray(a.scenes[id.scene], id, h.seed, rng, &o, &d);
+        w.ray_o[p] = make_float4(o.x, o.y, o.z, 0.0f);
+        w.ray_d[p] = make_float4(d.x, d.y, d.z, 0.0f);
+        w.thr[p] = make_float4(1.0f, 1.0f, 1.0f, __int_as_float(1));
+        w.meta[p] = make_uint4(uint32_t(id.scene), id.pixel, id.sample, rng.ctr);
     }
 }
 
@@ -646,16 +541,15 @@ __global__ void k_adj_ltot(RenderArgs a) {
 // 15.8 uncapped (up to 115 registers), 15.6 at 80, 17.1 at 64.
 constexpr int kShadeRegs = 96;
 
-template <int KIND, bool ADJ = false>
+// RECORD: the forward pass of the adjoint.
+template <int KIND, bool RECORD = false>
 __global__ void __maxnreg__(kShadeRegs) k_wf_shade(RenderArgs a, int b) {
-    extern __shared__ double adj_sh[];  // ADJ only: gradient block sums
     const WfBuffers& w = a.wf;
     const int n = w.cnt[b * kCntStride + 3 + KIND];
     int* next = w.cnt + (b + 1) * kCntStride;
     const int* q = w.q_mat[KIND];
     const int nb = (b + 1) & 1;
     const uint64_t seed = a.header->seed;
-    if (ADJ) adj_shared_zero(adj_sh, a.adj);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int p = q[i];
         uint4 meta = w.meta[p];
@@ -673,19 +567,14 @@ __global__ void __maxnreg__(kShadeRegs) k_wf_shade(RenderArgs a, int b) {
         rng.key = path_key(seed, meta.x, meta.y, meta.z);
         rng.ctr = meta.w;
         const VertexPlan pl = plan_vertex<KIND>(S, si, f3(tw), (__float_as_int(tw.w) & 1) != 0, b, rng);
-        bool adj_live = false;
-        if (ADJ) {
-            adj_live = adj_vertex_begin(a, adj_sh, S, si, pl, tw, p, meta.y);
-        } else if (!is_zero(pl.emit)) {
+        if (!is_zero(pl.emit)) {
             float4 L = w.L[p];
             L.x += pl.emit.x;
             L.y += pl.emit.y;
             L.z += pl.emit.z;
             w.L[p] = L;
         }
-        // the adjoint drops a path that carries no gradient
-        const bool live = !ADJ || adj_live;
-        const bool cont = live && pl.cont && (b + 1 < S.max_depth);
+        const bool cont = pl.cont && (b + 1 < S.max_depth);
         if (pl.shadow || pl.mis || cont) w.ray_o[p] = make_float4(si.P.x, si.P.y, si.P.z, 0.0f);
         if (pl.shadow) {
             w.sh_d[p] = make_float4(pl.sdir.x, pl.sdir.y, pl.sdir.z, pl.stmax);
@@ -693,7 +582,7 @@ __global__ void __maxnreg__(kShadeRegs) k_wf_shade(RenderArgs a, int b) {
         }
         // only MIS rays that meet their light are traced (mis_light_hit)
         bool mocc = false;
-        if (pl.mis && live) {
+        if (pl.mis) {
             float4 mh = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             mocc = mis_light_hit(S, ray_prep(si.P, pl.mdir, kRayEps, kFloatMax), pl.mlight, &mh);
             if (mocc) {
@@ -710,20 +599,100 @@ __global__ void __maxnreg__(kShadeRegs) k_wf_shade(RenderArgs a, int b) {
         meta.w = rng.ctr;
         w.meta[p] = meta;
         // a shadow ray whose contribution is zero in every channel adds
-        // nothing to Ls whatever its outcome (the adjoint still needs it: its
-        // radiance derivative need not be zero)
-        const int s_slot = warp_append(next + 2, live && pl.shadow != 0 && (ADJ || !is_zero(pl.scontrib)));
+        // nothing to Ls whatever its outcome (for the adjoint its radiance
+        // derivative has to be zero as well)
+        const int s_slot = warp_append(next + 2, pl.shadow != 0 && (!is_zero(pl.scontrib) || (RECORD && !is_zero(pl.sx))));
         if (s_slot >= 0) w.q_shadow[nb][s_slot] = p;
         const int o_slot = warp_append(next + 11, mocc);
         if (o_slot >= 0) w.q_mocc[nb][o_slot] = p;
         const int c_slot = warp_append(next + 0, cont);
         if (c_slot >= 0) w.q_cont[nb][c_slot] = p;
-        if (ADJ) {
-            const int v_slot = warp_append(next + 10, adj_live);
-            if (v_slot >= 0) a.adj.q_vtx[b & 1][v_slot] = p;
-        }
     }
-    if (ADJ) adj_shared_flush(adj_sh, a.adj);
+}
+
+// The replay of the vertices of bounce b (one shade queue of the forward pass):
+// the path's state is shaded again as k_wf_shade does, and what its shadow and
+// MIS rays found is taken from the records, so that a vertex's gradients are
+// complete at once (A, B and the radiance R = Ltot - acc - A - B of the vertices
+// after it give the texel, roughness and radiance terms of adjoint.cuh).  A path
+// that carries no gradient (total not finite, zero weight) is left out at every
+// vertex.  Bound as k_wf_shade is; 96 registers take as long as 128 and 80 (512 x
+// 512, 32 samples, depth 6: 7.21, 7.33 and 7.21 ms the whole backward call).
+template <int KIND>
+__global__ void __maxnreg__(kShadeRegs) k_adj_replay(RenderArgs a, int b) {
+    extern __shared__ double sh[];  // gradient block sums
+    const WfBuffers& w = a.wf;
+    const AdjBufs& A = a.adj;
+    const int n = w.cnt[b * kCntStride + 3 + KIND];
+    const int* q = w.q_mat[KIND];
+    const uint64_t seed = a.header->seed;
+    adj_shared_zero(sh, A);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int p = q[i];
+        uint4 meta = w.meta[p];
+        const float3 delta = adj_delta(A, meta.y);
+        const float3 Ltot = f3(A.Ltot[p]);
+        if (!finite3(Ltot) || is_zero(delta)) continue;
+        const SceneD& S = a.scenes[meta.x];
+        const float3 o = f3(w.ray_o[p]), d = f3(w.ray_d[p]);
+        const float4 h4 = w.hit[p];
+        HitD hit;
+        hit.t = h4.x;
+        hit.slot = __float_as_int(h4.y);
+        hit.u = h4.z;
+        hit.v = h4.w;
+        const SurfaceD si = surface_at(S, o, d, hit);
+        const float4 tw = w.thr[p];
+        const bool ce = (__float_as_int(tw.w) & 1) != 0;
+        Rng rng;
+        rng.key = path_key(seed, meta.x, meta.y, meta.z);
+        rng.ctr = meta.w;
+        const VertexPlan pl = plan_vertex<KIND>(S, si, f3(tw), ce, b, rng);
+        const bool cont = pl.cont && (b + 1 < S.max_depth);
+        if (cont) {
+            w.ray_o[p] = make_float4(si.P.x, si.P.y, si.P.z, 0.0f);
+            w.ray_d[p] = make_float4(pl.cdir.x, pl.cdir.y, pl.cdir.z, 0.0f);
+            w.thr[p] = make_float4(pl.T.x, pl.T.y, pl.T.z, __int_as_float(pl.count_emission));
+            meta.w = rng.ctr;
+            w.meta[p] = meta;
+        }
+        if (si.light >= 0 && si.light < A.nlight && ce && can_emit(S.lights[si.light], si.wi, si.Ns))
+            adj_radiance(sh, A, si.light, delta * f3(tw));
+        float3 Av = splat3(0.0f), Bv = splat3(0.0f);
+        if (pl.shadow && (!is_zero(pl.scontrib) || !is_zero(pl.sx)) && a.rec_shadow[p]) {
+            Av = pl.scontrib;
+            if (pl.slight < A.nlight) adj_radiance(sh, A, pl.slight, delta * pl.sx);
+        }
+        float4 mh = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (pl.mis && mis_light_hit(S, ray_prep(si.P, pl.mdir, kRayEps, kFloatMax), pl.mlight, &mh) && a.rec_mis[p]) {
+            float3 X = splat3(0.0f);
+            Bv = mis_add(S, si.P, pl.mdir, mh, f3(tw), pl.mfactor, pl.mpdf, &X);
+            if (__float_as_int(mh.y) >= 0 && pl.mlight >= 0 && pl.mlight < A.nlight) adj_radiance(sh, A, pl.mlight, delta * X);
+        }
+        const float4 acc4 = A.acc[p];
+        const float3 acc = f3(acc4) + pl.emit;
+        const float3 after = Ltot - acc - Av - Bv;
+        const MaterialD& m = S.materials[si.material];
+        if (m.type == BSDF_LAMBERTIAN && m.albedo_tex >= 0) {
+            const TextureD& tex = S.textures[m.albedo_tex];
+            const float3 alb = texture_rgb(tex, si.uvw);
+            const float3 num = delta * (Av + Bv + after);
+            double* g = A.g_tex + A.tex_offset[m.albedo_tex] + 3 * texel_index(tex, si.uvw);
+            if (alb.x > 0.0f && num.x != 0.0f) atomicAdd(g + 0, double(num.x / alb.x));
+            if (alb.y > 0.0f && num.y != 0.0f) atomicAdd(g + 1, double(num.y / alb.y));
+            if (alb.z > 0.0f && num.z != 0.0f) atomicAdd(g + 2, double(num.z / alb.z));
+        }
+        if (m.type == BSDF_CONDUCTOR || m.type == BSDF_DIELECTRIC_GGX) {
+            float gr = 0.0f;
+            if (!is_zero(Av)) gr += dot(delta, Av) * dlogf_droughness(m, si.wi, pl.sdir, si.Ns);
+            if (!is_zero(Bv)) gr += dot(delta, Bv) * dlogf_droughness(m, si.wi, pl.mdir, si.Ns);
+            if (pl.cont) gr += dot(delta, after) * dlogf_droughness(m, si.wi, pl.cdir, si.Ns);
+            adj_add(sh, si.material, double(gr));
+        }
+        const float3 nacc = acc + (Av + Bv);
+        A.acc[p] = make_float4(nacc.x, nacc.y, nacc.z, 0.0f);
+    }
+    adj_shared_flush(sh, A);
 }
 
 // FP64 accumulation of one batch into the scenes' films.  With the default
@@ -1006,7 +975,6 @@ RenderArgs make_args(cgpu_ctx* ctx) {
     a.films = ctx->d_films;
     a.wf = ctx->wf;
     a.counters = ctx->d_counters;
-    a.adj = AdjBufs{};
     a.sorted = nullptr;
     a.refill_closest = refill_lanes(ctx->tuning.refill_closest);
     a.refill_any = refill_lanes(ctx->tuning.refill_any);
@@ -1059,8 +1027,11 @@ bool large_batch(const cgpu_ctx* ctx, uint64_t paths) { return std::min<uint64_t
 // An empty launch still costs 2 to 4 us between two passes (Cornell box, 256 x
 // 256, 16 samples, depth 6: 1.28 -> 1.20 ms without four of them a bounce).
 uint32_t launch_shade(cgpu_ctx* ctx, const RenderArgs& a, int b, const int (&grid)[kNumBsdfKinds]) {
-    static void (*const kernel[kNumBsdfKinds])(RenderArgs, int) = {k_wf_shade<0>, k_wf_shade<1>, k_wf_shade<2>, k_wf_shade<3>,
-                                                                   k_wf_shade<4>};
+    static void (*const plain[kNumBsdfKinds])(RenderArgs, int) = {k_wf_shade<0>, k_wf_shade<1>, k_wf_shade<2>, k_wf_shade<3>,
+                                                                  k_wf_shade<4>};
+    static void (*const record[kNumBsdfKinds])(RenderArgs, int) = {k_wf_shade<0, true>, k_wf_shade<1, true>, k_wf_shade<2, true>,
+                                                                   k_wf_shade<3, true>, k_wf_shade<4, true>};
+    auto& kernel = a.rec_shadow ? record : plain;
     uint32_t launches = 0;
     for (int k = 0; k < kNumBsdfKinds; ++k) {
         if (!(ctx->batch_kinds >> k & 1u)) continue;
@@ -1071,7 +1042,11 @@ uint32_t launch_shade(cgpu_ctx* ctx, const RenderArgs& a, int b, const int (&gri
 }
 
 // Enqueue the wavefront schedule for one batch on ctx->stream.
-cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool splat, bool counting) {
+void set_records(RenderArgs& a, const AdjRecords& r, int b, int outcomes);
+
+// rec (optional): the batch's rays are recorded there, for the adjoint.
+cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool splat, bool counting,
+                              const AdjRecords* rec = nullptr) {
     RenderArgs a = make_args(ctx);
     // With per-kernel timing on, the shadow pass runs after the extend pass on
     // the same stream, so that each event pair brackets one kernel alone.
@@ -1117,6 +1092,7 @@ cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool spl
                                     grid_for(ctx, k_wf_shade<2>, bs, paths), grid_for(ctx, k_wf_shade<3>, bs, paths),
                                     grid_for(ctx, k_wf_shade<4>, bs, paths)};
     for (int b = 0; b <= depth; ++b) {
+        if (rec) set_records(a, *rec, b, b - 1);
         cudaEventRecord(fork, s);
         cudaStreamWaitEvent(side, fork, 0);
         if (reorder && b > 0) {
@@ -1234,8 +1210,7 @@ void cg_free_render_state(cgpu_ctx* ctx) {
         cudaFree(ctx->adj_block);
         ctx->adj_block = nullptr;
     }
-    ctx->adj = AdjBufs{};
-    ctx->adj_cap = 0;
+    ctx->adj_bytes = 0;
     if (ctx->sort_block) {
         cudaFree(ctx->sort_block);
         ctx->sort_block = nullptr;
@@ -1311,7 +1286,7 @@ cgpu_status cg_render_batches(cgpu_ctx* ctx, const cgpu_render_params* p) {
             c.sample0 = next[i];
             c.nsamples = k;
             c.pix_begin = pix;
-            c.pad = 0;
+            c.pixel0 = 0;
             used += k * npix;
             pix += npix;
             next[i] += k;
@@ -1481,88 +1456,76 @@ cgpu_status cg_film_clear(cgpu_ctx* ctx, int scene) {
 }
 
 // ======================================================= wavefront adjoint ==
-// cgpu_adjoint_backward on the wavefront schedule.  Per batch of whole
-// samples of the scene: (A) the forward wavefront render of the batch without
-// the film splat, whose per-path radiance is the Ltot of each path; (B) the
-// same paths regenerated and replayed pass by pass with the adjoint variants
-// of the kernels (extend / shadow store the MIS and shadow outcomes instead of
-// adding them; shade keeps each vertex's state and queues it), and after each
-// traversal pass the gradient kernel of the vertices whose rays it traced.
+// cgpu_adjoint_backward on the wavefront schedule.  Per batch: (A) the forward
+// wavefront render without the film splat, whose per-path radiance is the Ltot
+// of each path and whose passes record what every ray found; (B) the same paths
+// shaded again bounce by bounce from the records (k_adj_replay), without a ray:
+// 26 bytes a path and bounce with two kinds of material.  With the rays of (B)
+// traced again, each vertex's terms kept for a kernel behind them (120 bytes a
+// path), the backward call of 512 x 512 pixels, 32 samples, depth 6 took 12.3 ms,
+// now 7.2; of 127 x 95, 8 samples, depth 4 1.20 and 0.75.
 namespace {
 
-void enqueue_adjoint_pass(cgpu_ctx* ctx, const RenderArgs& a, int depth, uint32_t paths, size_t shared_bytes) {
-    cudaStream_t s = ctx->stream, side = ctx->side;
-    cudaEvent_t fork = nullptr, join = nullptr;
-    cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
-    cudaMemsetAsync(ctx->wf.cnt, 0, size_t(depth + 2) * kCntStride * sizeof(int), s);
-    const int bt = ctx->tuning.block_trace, bs = ctx->tuning.block_shade;
-    const bool sph = ctx->batch_spheres;
-    // the persistent passes when the tuning uses them (traversal 2 / 3), else the per-ray loops
-    const int trav = ctx->batch_closest, trav_any = ctx->batch_any;
-    auto ext = trav >= 2 ? (sph ? k_wf_extend_pww<false, true> : k_wf_extend_pww<false, false>)
-                         : (sph ? k_wf_extend<false, true> : k_wf_extend<false, false>);
-    auto shd = trav_any == 3 ? (sph ? k_wf_shadow_pww<false, true, true> : k_wf_shadow_pww<false, false, true>)
-                         : (sph ? k_wf_shadow<false, true, true> : k_wf_shadow<false, false, true>);
-    auto mo = sph ? k_wf_mis_occl<false, true, true> : k_wf_mis_occl<false, false, true>;
-    auto ties = sph ? k_wf_ties<false, true> : k_wf_ties<false, false>;
-    void (*shade[kNumBsdfKinds])(RenderArgs, int) = {k_wf_shade<0, true>, k_wf_shade<1, true>, k_wf_shade<2, true>,
-                                                     k_wf_shade<3, true>, k_wf_shade<4, true>};
-    k_wf_generate<<<grid_for(ctx, k_wf_generate, kBlock, paths), kBlock, 0, s>>>(a);
-    const size_t ext_sm = stack_smem(ext, trav >= 2, true, bt), sh_sm = stack_smem(shd, trav_any == 3, false, bt);
-    const int gext = grid_for(ctx, ext, bt, paths, ext_sm), gsh = grid_for(ctx, shd, bt, paths, sh_sm);
-    const int gmo = grid_for(ctx, mo, bt, paths), gties = grid_for(ctx, ties, kTieBlock, paths);
-    const int gv = grid_for(ctx, k_adj_vertex, kBlock, paths, shared_bytes);
-    int gsd[kNumBsdfKinds];
-    for (int k = 0; k < kNumBsdfKinds; ++k) gsd[k] = grid_for(ctx, shade[k], bs, paths, shared_bytes);
-    uint32_t launches = 1;
-    for (int b = 0; b <= depth; ++b) {
-        cudaEventRecord(fork, s);
-        cudaStreamWaitEvent(side, fork, 0);
-        ext<<<gext, bt, ext_sm, s>>>(a, b);
-        if (trav >= 2) {
-            ties<<<gties, kTieBlock, 0, s>>>(a, b);
-            launches += 1;
-        }
-        shd<<<gsh, bt, sh_sm, side>>>(a, b);
-        if (b > 0) {
-            mo<<<gmo, bt, 0, side>>>(a, b);
-            launches += 1;
-        }
-        cudaEventRecord(join, side);
-        cudaStreamWaitEvent(s, join, 0);
-        launches += 2;
-        if (b > 0) {
-            k_adj_vertex<<<gv, kBlock, shared_bytes, s>>>(a, b - 1);
-            launches += 1;
-        }
-        if (b == depth) break;
-        for (int k = 0; k < kNumBsdfKinds; ++k)
-            if (ctx->batch_kinds >> k & 1u) {
-                shade[k]<<<gsd[k], bs, shared_bytes, s>>>(a, b);
-                ++launches;
-            }
-    }
-    cudaEventDestroy(fork);
-    cudaEventDestroy(join);
-    ctx->stats.kernel_launches += launches;
+// Most bytes of records a batch takes: 13 million paths of depth 12 through three
+// kinds of material.  Beyond that the frame is done in parts.
+constexpr uint64_t kAdjRecordBytes = uint64_t(4) << 30;
+
+// The launches of bounce b of a batch with records: hits and shade queues are
+// the row's own, and so are the outcomes of the rays that the shadow and MIS
+// passes of row `outcomes` trace.
+void set_records(RenderArgs& a, const AdjRecords& r, int b, int outcomes) {
+    const size_t row = size_t(std::min(std::max(b, 0), r.depth - 1)) * r.stride;
+    const size_t out = size_t(std::min(std::max(outcomes, 0), r.depth - 1)) * r.stride;
+    a.wf.hit = r.hit + row;
+    for (int k = 0; k < kNumBsdfKinds; ++k)
+        if (r.q_mat[k]) a.wf.q_mat[k] = r.q_mat[k] + row;
+    a.rec_shadow = r.shadow + out;
+    a.rec_mis = r.mis + out;
 }
 
-cgpu_status ensure_adj_buffers(cgpu_ctx* ctx) {
-    if (ctx->adj_cap >= ctx->path_cap && ctx->adj_block) return CGPU_OK;
-    if (ctx->adj_block) cudaFree(ctx->adj_block);
-    ctx->adj_block = nullptr;
-    ctx->adj_cap = 0;
-    AdjBufs tmp{};
-    const size_t bytes = adj_layout(nullptr, ctx->path_cap, &tmp);
-    cudaError_t e = cudaMalloc(&ctx->adj_block, bytes);
-    if (e != cudaSuccess) {
-        ctx->adj_block = nullptr;
-        return cg_fail(ctx, CGPU_ERR_OUT_OF_MEMORY, "adjoint buffers: " + std::string(cudaGetErrorString(e)));
+void enqueue_adjoint_replay(cgpu_ctx* ctx, RenderArgs a, const AdjRecords& rec, int depth, uint32_t paths, size_t shared_bytes) {
+    cudaStream_t s = ctx->stream;
+    static void (*const replay[kNumBsdfKinds])(RenderArgs, int) = {k_adj_replay<0>, k_adj_replay<1>, k_adj_replay<2>,
+                                                                   k_adj_replay<3>, k_adj_replay<4>};
+    const int bs = ctx->tuning.block_shade;
+    k_adj_begin<<<grid_for(ctx, k_adj_begin, kBlock, paths), kBlock, 0, s>>>(a);
+    int grid[kNumBsdfKinds];
+    for (int k = 0; k < kNumBsdfKinds; ++k) grid[k] = grid_for(ctx, replay[k], bs, paths, shared_bytes);
+    ctx->stats.kernel_launches += 1;
+    for (int b = 0; b < depth; ++b) {
+        set_records(a, rec, b, b);
+        for (int k = 0; k < kNumBsdfKinds; ++k)
+            if (ctx->batch_kinds >> k & 1u) {
+                replay[k]<<<grid[k], bs, shared_bytes, s>>>(a, b);
+                ctx->stats.kernel_launches += 1;
+            }
     }
-    adj_layout(static_cast<char*>(ctx->adj_block), ctx->path_cap, &ctx->adj);
-    ctx->adj_cap = ctx->path_cap;
-    return CGPU_OK;
+}
+
+// Room for the adjoint state of *paths paths, kept between calls.  Where the
+// device has not that much left, *paths is halved until it has.
+cgpu_status ensure_adj_buffers(cgpu_ctx* ctx, int depth, uint32_t* paths, AdjBufs* a, AdjRecords* r) {
+    cudaError_t e = cudaSuccess;
+    for (uint32_t n = *paths;; n = (n + 1) / 2) {
+        const size_t bytes = adj_layout(nullptr, n, ctx->batch_kinds, depth, a, r);
+        e = cudaSuccess;
+        if (bytes > ctx->adj_bytes) {
+            if (ctx->adj_block) cudaFree(ctx->adj_block);
+            ctx->adj_block = nullptr;
+            ctx->adj_bytes = 0;
+            e = cudaMalloc(&ctx->adj_block, bytes);
+            if (e == cudaSuccess) ctx->adj_bytes = bytes;
+            else ctx->adj_block = nullptr;
+        }
+        if (e == cudaSuccess) {
+            *paths = n;
+            adj_layout(static_cast<char*>(ctx->adj_block), n, ctx->batch_kinds, depth, a, r);
+            return CGPU_OK;
+        }
+        cudaGetLastError();
+        if (e != cudaErrorMemoryAllocation || n <= 4096) break;
+    }
+    return cg_fail(ctx, CGPU_ERR_OUT_OF_MEMORY, "adjoint buffers: " + std::string(cudaGetErrorString(e)));
 }
 
 }  // namespace
@@ -1576,56 +1539,55 @@ cgpu_status cg_adjoint_wavefront(cgpu_ctx* ctx, int scene, uint32_t spp, uint64_
     if (st != CGPU_OK) return st;
     st = ensure_path_buffers(ctx, paths_capacity(ctx, npix), sl.max_depth);
     if (st != CGPU_OK) return st;
-    st = ensure_adj_buffers(ctx);
-    if (st != CGPU_OK) return st;
+    const int depth = sl.max_depth;
     const size_t shared_bytes = size_t(params.nmat + 3 * params.nlight) * sizeof(double);
-    if (shared_bytes > 48 * 1024) {
-        const int sb = int(shared_bytes);
-        cudaFuncSetAttribute(k_adj_vertex, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
-        cudaFuncSetAttribute(k_wf_shade<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
-        cudaFuncSetAttribute(k_wf_shade<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
-        cudaFuncSetAttribute(k_wf_shade<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
-        cudaFuncSetAttribute(k_wf_shade<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
-        cudaFuncSetAttribute(k_wf_shade<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
-    }
     RenderArgs a = make_args(ctx);
     a.adj = params;
-    a.adj.Ltot = ctx->adj.Ltot;
-    a.adj.acc = ctx->adj.acc;
-    a.adj.st_a = ctx->adj.st_a;
-    a.adj.st_b = ctx->adj.st_b;
-    a.adj.st_c = ctx->adj.st_c;
-    a.adj.mis_B = ctx->adj.mis_B;
-    a.adj.mis_X = ctx->adj.mis_X;
-    a.adj.q_vtx[0] = ctx->adj.q_vtx[0];
-    a.adj.q_vtx[1] = ctx->adj.q_vtx[1];
+    // a batch: whole samples of the frame or, where the records of one sample
+    // take more than kAdjRecordBytes, parts of one
+    const uint64_t want = std::min<uint64_t>({ctx->path_cap, uint64_t(spp) * npix,
+                                              std::max<uint64_t>(1, kAdjRecordBytes / adj_record_bytes(sl.kinds, depth))});
+    uint32_t room = uint32_t(want);
+    AdjRecords rec;
+    st = ensure_adj_buffers(ctx, depth, &room, &a.adj, &rec);
+    if (st != CGPU_OK) return st;
+    if (shared_bytes > 48 * 1024) {
+        const int sb = int(shared_bytes);
+        cudaFuncSetAttribute(k_adj_replay<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+        cudaFuncSetAttribute(k_adj_replay<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+        cudaFuncSetAttribute(k_adj_replay<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+        cudaFuncSetAttribute(k_adj_replay<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+        cudaFuncSetAttribute(k_adj_replay<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+    }
     ctx->stats = cgpu_render_stats{};
     const bool persistent = sl.d.num_tris >= kSmallScene && large_batch(ctx, uint64_t(spp) * npix);
     choose_traversal(ctx, persistent, persistent);
-    const uint32_t per = std::max<uint32_t>(1, ctx->path_cap / npix);
-    const int depth = sl.max_depth;
-    for (uint32_t done = 0; done < spp;) {
+    const uint32_t per = std::max<uint32_t>(1, room / npix), part = std::min(room, npix);
+    for (uint32_t done = 0, pixel0 = 0; done < spp;) {
+        const uint32_t pixels = std::min(part, npix - pixel0);
         const uint32_t k = std::min(per, spp - done);
-        const uint32_t paths = k * npix;
+        const uint32_t paths = k * pixels;
         cudaStreamSynchronize(ctx->stream);
-        ctx->h_chunks[0] = Chunk{scene, 0, npix, uint32_t(sl.width), done, k, 0, 0};
+        ctx->h_chunks[0] = Chunk{scene, 0, pixels, uint32_t(sl.width), done, k, 0, pixel0};
         BatchHeader& h = *ctx->h_header;
         h.num_chunks = 1;
         h.total_paths = paths;
-        h.total_pixels = npix;
+        h.total_pixels = pixels;
         h.max_depth = depth;
         h.seed = seed;
         cudaMemcpyAsync(ctx->d_chunks, ctx->h_chunks, sizeof(Chunk), cudaMemcpyHostToDevice, ctx->stream);
         cudaMemcpyAsync(ctx->d_header, ctx->h_header, sizeof(BatchHeader), cudaMemcpyHostToDevice, ctx->stream);
-        st = enqueue_wavefront(ctx, depth, paths, false, false);
+        st = enqueue_wavefront(ctx, depth, paths, false, false, &rec);
         if (st != CGPU_OK) return st;
-        k_adj_ltot<<<grid_for(ctx, k_adj_ltot, 256, paths), 256, 0, ctx->stream>>>(a);
-        ctx->stats.kernel_launches += 1;
-        enqueue_adjoint_pass(ctx, a, depth, paths, shared_bytes);
+        enqueue_adjoint_replay(ctx, a, rec, depth, paths, shared_bytes);
         st = cg_cuda(ctx, cudaGetLastError(), "adjoint wavefront launch");
         if (st != CGPU_OK) return st;
         ctx->stats.batches += 1;
-        done += k;
+        pixel0 += pixels;
+        if (pixel0 == npix) {
+            pixel0 = 0;
+            done += k;
+        }
     }
     ctx->stats.paths = uint64_t(spp) * npix;
     collect_profile(ctx);  // the forward passes' events, with profiling on
