@@ -438,11 +438,14 @@ CG_D bool visit_leaf(const SceneD& S, const RayPre& r, uint32_t e, float& tcur, 
 // megakernel's traversal (its threads are at different bounces anyway) and
 // every any-hit query (the first hit ends the walk, so there is nothing to
 // gain from holding leaves back).
+// Nodes that end before `near` are left out, and hits beyond `far`.
 template <bool ANY, bool COUNT, bool SPH = true>
-CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* cnt) {
+CG_D bool traverse(const SceneD& S, const RayPre& r, float near, float far, HitD* hit, TraceCounters* cnt) {
     LocalStack stack;
     int sp = 0;
-    float tcur = r.tmax;
+    RayPre box = r;
+    box.tmin = near;
+    float tcur = far;
     int hslot = -1;
     float hu = 0.0f, hv = 0.0f;
     uint32_t cur = 0;  // root first (always an inner node)
@@ -457,7 +460,7 @@ CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* c
                 return true;
             }
         } else {
-            next = visit_node<ANY, COUNT>(S, r, cur, tcur, stack, sp, cnt);
+            next = visit_node<ANY, COUNT>(S, box, cur, tcur, stack, sp, cnt);
         }
         // else the next stack entry that can still hold a closer hit
         while (next == kNoEntry && sp > 0) {
@@ -472,6 +475,11 @@ CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* c
     hit->u = hu;
     hit->v = hv;
     return hslot >= 0;
+}
+
+template <bool ANY, bool COUNT, bool SPH = true>
+CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* cnt) {
+    return traverse<ANY, COUNT, SPH>(S, r, r.tmin, r.tmax, hit, cnt);
 }
 
 // Whether a primitive other than `prim_l` comes before the hit (t_l, prim_l,

@@ -149,3 +149,47 @@ def test_query_batches_match_small_queries(gpu_ctx, name):
         for j in range(len(whole[q])):
             assert np.array_equal(whole[q][j], np.concatenate([p[q][j] for p in parts])), (name, q, j)
     gpu_ctx.release(sid)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layers,step", [(2, 0.0), (3, 0.0), (3, 1e-3), (7, 5e-4)])
+def test_layers_within_the_tie_window(gpu_ctx, layers, step):
+    """Several primitives within the tie window (2^-16 of the scene's 560 units)
+    of every hit on a tilted sheet: the nearest is traced again within its
+    window.  Render against the megakernel, a large batch of queries (hits
+    before and behind the origin, t_max on the sheet) against small ones."""
+    s = scenes.cornell_box(48, 40, 4, 4)
+    m = 24
+    u, v = np.meshgrid(np.linspace(60, 500, m), np.linspace(60, 500, m), indexing="ij")
+    g = np.stack([u, v, 150.0 + 0.3 * u - 0.2 * v], -1)
+    quads = np.concatenate([np.stack([g[:-1, :-1], g[1:, :-1], g[1:, 1:]], 2).reshape(-1, 3, 3),
+                            np.stack([g[:-1, :-1], g[1:, 1:], g[:-1, 1:]], 2).reshape(-1, 3, 3)])
+    tri = np.concatenate([quads + [0, 0, step * k] for k in range(layers)]).astype(np.float32)
+    s.primitives.append(scenes.TriangleMesh(name="sheet", material=s.materials[1].name, positions=tri))
+    sid = gpu_ctx.upload(abi.flatten(s))
+    base = gpu_ctx.tuning()
+    films = []
+    try:
+        gpu_ctx.set_tuning(64, 64, 0, traversal=3)
+        for mode in (CGPU_MODE_MEGAKERNEL, CGPU_MODE_WAVEFRONT):
+            gpu_ctx.film_clear(sid)
+            gpu_ctx.render([sid], 0, 4, seed=8, mode=mode)
+            films.append(gpu_ctx.film_read(sid))
+        for x, y in zip(*films):
+            assert np.array_equal(x, y)
+        n = (1 << 17) + 5
+        rng = np.random.default_rng(layers)
+        rays = np.zeros((n, 8), np.float32)
+        rays[:, :3] = rng.uniform(50, 510, (n, 3))
+        rays[:, 4:7] = rng.normal(0, 1, (n, 3))
+        rays[:, 3], rays[:, 7] = 1e-3, 3.4e38
+        rays[:n // 3, 3] = -1000.0
+        rays[n // 3:n // 2, 7] = gpu_ctx.trace_closest(sid, rays[n // 3:n // 2])[1]
+        whole = gpu_ctx.trace_closest(sid, rays)
+        assert (whole[0] >= 0).mean() > 0.5 and (whole[1] < 0).any()
+        parts = [gpu_ctx.trace_closest(sid, rays[i:i + 4000]) for i in range(0, n, 4000)]
+        for j in range(len(whole)):
+            assert np.array_equal(whole[j], np.concatenate([p[j] for p in parts])), j
+    finally:
+        gpu_ctx.set_tuning_dict(base)
+        gpu_ctx.release(sid)
