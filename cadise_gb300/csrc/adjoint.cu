@@ -10,8 +10,9 @@
 // A path's radiance is a sum of terms (emission, NEE light sample, NEE BSDF
 // sample) at each vertex j, and every later term carries the continuation
 // weight f_j cos / pdf of vertex j.  Each path is replayed twice from its
-// seed (no stored vertices): replay 1 gives the total L; replay 2 walks the
-// vertices again with R_j = L - (terms so far), the radiance still to come:
+// seed: replay 1 gives the total L (and, on the wavefront schedule, records what
+// its rays found); replay 2 walks the vertices again with
+// R_j = L - (terms so far), the radiance still to come:
 //   albedo texel at a Lambert vertex j:  dL += delta * (A_j + B_j + R_j) / albedo_j
 //   roughness of vertex j's material:   dL += delta . (A_j g(w_l) + B_j g(w_b) + R_j g(w_c)),
 //                                        g = d ln f / d roughness

@@ -9,8 +9,9 @@
 // counter-based random stream keyed by (seed, scene, pixel, sample).
 //
 // Wavefront schedule of one batch (replayed as one CUDA graph):
-//   generate -> for b in [0, max_depth): { extend(b) || shadow(b) ; shade_k(b) for each BSDF kind }
-//            -> extend(max_depth) || shadow(max_depth) -> splat
+//   generate -> for b in [0, max_depth): { extend(b), ties(b) || shadow(b), mis_occl(b) ;
+//               shade_k(b) for each BSDF kind that the scenes have }
+//            -> extend(max_depth) .. mis_occl(max_depth) -> splat
 // Queues hold path ids; per-path state lives in SoA arrays indexed by path.
 // Queue appends are warp-aggregated (ballot / match + one atomic per group).
 #include "film.cuh"

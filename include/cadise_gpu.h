@@ -440,8 +440,8 @@ cgpu_status cgpu_adjoint_backward(cgpu_ctx* ctx, int32_t scene, uint32_t spp, ui
                                   const float* d_loss_d_image, double* grad_texels, double* grad_roughness,
                                   double* grad_radiance);
 /* Schedule of cgpu_adjoint_backward: CGPU_MODE_WAVEFRONT (default; a forward
- * wavefront pass for each path's radiance, then a wavefront replay with a
- * gradient kernel after each traversal pass) or CGPU_MODE_MEGAKERNEL (one
+ * wavefront pass for each path's radiance that records what its rays found,
+ * then a wavefront replay from the records) or CGPU_MODE_MEGAKERNEL (one
  * thread replays one path twice).  Both compute the same estimator on the
  * same path samples; they differ in FP64 summation order only. */
 cgpu_status cgpu_set_adjoint_mode(cgpu_ctx* ctx, int32_t mode);
