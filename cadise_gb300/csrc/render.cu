@@ -319,7 +319,7 @@ __global__ void k_wf_extend_dyn(RenderArgs a, int b) {
 }
 
 // Registers of the persistent passes: 18 blocks of 64 threads an SM.  The
-// 1 M-triangle frame's closest-hit passes take 33.9 ms at 56 registers (20 bytes
+// 1 M-triangle frame's closest-hit passes take 33.9 ms at 56 registers (32 bytes
 // of spills in the ray set-up), 34.6 at 64 and 37.3 at 48.
 constexpr int kPersistRegs = 56;
 
