@@ -706,6 +706,11 @@ __global__ void __maxnreg__(kShadeRegs) k_adj_replay(RenderArgs a, int b) {
 // box filter of size 1 a sample at (ix + fx, iy + fy) lands in pixel (ix, iy)
 // only; other filters go through splat_filtered.  NaN / Inf samples are
 // dropped as FilmTile::addSample does (source/core/film/filmTile.cpp:21-28).
+// One warp a block: a filtered frame of 333 x 251 pixels is 327 blocks of 256
+// threads, three on some SMs and two on the others (0.68 ms; 0.59 in blocks of
+// 128, 0.54 of 64, 0.53 of 32; a 1080p frame 0.66 in any).
+constexpr int kSplatBlock = 32;
+
 __global__ void k_splat(RenderArgs a) {
     const BatchHeader h = *a.header;
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < h.total_pixels; idx += gridDim.x * blockDim.x) {
@@ -1131,8 +1136,8 @@ cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool spl
         timed(ctx, CGPU_KERNEL_SHADE, s, [&] { launches += launch_shade(ctx, a, b, gsd); });
     }
     if (splat) {
-        const int gsp = grid_for(ctx, k_splat, 256, ctx->h_header->total_pixels);
-        timed(ctx, CGPU_KERNEL_SPLAT, s, [&] { k_splat<<<gsp, 256, 0, s>>>(a); });
+        const int gsp = grid_for(ctx, k_splat, kSplatBlock, ctx->h_header->total_pixels);
+        timed(ctx, CGPU_KERNEL_SPLAT, s, [&] { k_splat<<<gsp, kSplatBlock, 0, s>>>(a); });
         launches += 1;
     }
     cudaEventDestroy(fork);
@@ -1157,8 +1162,8 @@ cgpu_status run_batch(cgpu_ctx* ctx, int mode, int depth, uint32_t paths, bool s
         }
         ctx->stats.kernel_launches += 1;
         if (splat) {
-            const int gsp = grid_for(ctx, k_splat, 256, ctx->h_header->total_pixels);
-            timed(ctx, CGPU_KERNEL_SPLAT, ctx->stream, [&] { k_splat<<<gsp, 256, 0, ctx->stream>>>(a); });
+            const int gsp = grid_for(ctx, k_splat, kSplatBlock, ctx->h_header->total_pixels);
+            timed(ctx, CGPU_KERNEL_SPLAT, ctx->stream, [&] { k_splat<<<gsp, kSplatBlock, 0, ctx->stream>>>(a); });
             ctx->stats.kernel_launches += 1;
         }
         return cg_cuda(ctx, cudaGetLastError(), "megakernel launch");
@@ -1678,7 +1683,7 @@ void enqueue_wavefront_serial(cgpu_ctx* ctx, const RenderArgs& a, int depth, uin
         if (b == depth) break;
         ctx->stats.kernel_launches += launch_shade(ctx, a, b, gsd);
     }
-    k_splat<<<grid_for(ctx, k_splat, 256, npix), 256, 0, s>>>(a);
+    k_splat<<<grid_for(ctx, k_splat, kSplatBlock, npix), kSplatBlock, 0, s>>>(a);
     ctx->stats.kernel_launches +=
         uint32_t(3 + 2 * (depth + 1) + depth + (trav >= 2 ? depth + 1 : 0));
 }
