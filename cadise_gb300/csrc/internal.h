@@ -207,17 +207,15 @@ struct RenderArgs {
 
 // Where the tuning leaves the traversal variant open (traversal 0), the
 // persistent passes take batches of kLargeBatch paths through scenes of
-// kSmallScene records or more, and any batch through kLargeScene records or more
-// (ms a frame of depth 8, one ray per thread / persistent: 2,457,600 paths
-// through 960 triangles 3.22 / 3.03, through 204,800 7.71 / 5.96; 12,288 paths
-// through 51,200 0.96 / 0.90, through 204,800 1.05 / 0.97).  Elsewhere the second
-// launch for the rays within the tie window costs what they save (Cornell box,
-// 36 triangles, 1,048,576 paths 1.20 / 1.24; 262,144 paths through 3,200
-// triangles 1.05 / 1.06; an adjoint iteration of 96,520 paths through 3,842
-// triangles 1.86 / 1.96).  The adjoint's passes, launched one by one, go by the
-// paths alone; the allocation-free render, on one stream, takes the any-hit pass
-// (1.09 / 1.05).
-constexpr int kSmallScene = 512, kLargeScene = 16384;
+// kSmallScene records or more (ms a frame of depth 8, one ray per thread /
+// persistent: 2,457,600 paths through 960 triangles 2.83 / 2.99, 3,200 3.78 / 3.73,
+// 12,800 4.33 / 4.05, 204,800 6.99 / 5.84; 921,600 through 102,400 2.75 / 2.51).
+// Elsewhere one ray per thread, whose three passes of a bounce are one launch, is
+// the faster one: 262,144 paths through 960 triangles 0.78 / 0.90, 204,800 1.45 /
+// 1.58; 12,288 paths 0.60 / 0.63 and 0.95 / 0.96; an adjoint iteration of 96,520
+// paths through 3,842 triangles 1.12 / 1.37; the allocation-free render 0.75 /
+// 1.05, always by that one.
+constexpr int kSmallScene = 2048;
 constexpr uint64_t kLargeBatch = 1u << 19;
 
 // The refill thresholds of a tuning, 0 replaced by the default.

@@ -386,8 +386,8 @@ typedef struct cgpu_tuning {
     int32_t block_shade;   /* threads per block: shade-by-BSDF kernels */
     uint32_t max_paths;    /* paths in flight per wavefront batch; 0 = automatic (2^21, at least one frame) */
     int32_t traversal;     /* 0: the library's choice by scene and batch size (default): 3 where its passes
-                              are the faster ones (scenes of 16,384 triangles, or of 512 in batches of 2^19
-                              paths), else one ray per thread per grid-stride step; 1: persistent warps that hand
+                              are the faster ones (batches of 2^19 paths through scenes of 2,048 triangles),
+                              else one ray per thread per grid-stride step; 1: persistent warps that hand
                               a finished lane the next ray at once; 2: persistent closest-hit pass that
                               votes between node and triangle steps and refills a warp's finished lanes
                               once fewer than refill_closest of its lanes still trace, any-hit with one
