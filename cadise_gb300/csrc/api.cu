@@ -106,6 +106,7 @@ cgpu_status cg_sync_tables(cgpu_ctx* ctx) {
     if (!ctx->tables_dirty) return CGPU_OK;
     const int n = int(ctx->scenes.size());
     if (n > ctx->table_cap) {
+        cg_drop_graphs(ctx);  // their launches hold the addresses of both tables
         if (ctx->d_scenes) cudaFree(ctx->d_scenes);
         if (ctx->d_films) cudaFree(ctx->d_films);
         ctx->d_scenes = nullptr;
