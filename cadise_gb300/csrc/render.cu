@@ -27,8 +27,12 @@
 
 namespace cg {
 
+// At 128 registers a quarter of an SM holds four warps, so that blocks of up to
+// 512 threads launch (uncapped the counting variants take 136: 384 threads).
+constexpr int kMegakernelRegs = 128;
+
 template <bool COUNT, bool SPH>
-__global__ void k_megakernel(RenderArgs a) {
+__global__ void __maxnreg__(kMegakernelRegs) k_megakernel(RenderArgs a) {
     const BatchHeader h = *a.header;
     TraceCounters tc{0, 0}, ta{0, 0};
     uint32_t nc = 0, na = 0;
