@@ -1091,9 +1091,15 @@ uint32_t launch_shade(cgpu_ctx* ctx, const RenderArgs& a, int b, const int (&gri
 // Enqueue the wavefront schedule for one batch on ctx->stream.
 void set_records(RenderArgs& a, const AdjRecords& r, int b, int outcomes);
 
+// The film splat of the batch in h_header.
+void launch_splat(cgpu_ctx* ctx, const RenderArgs& a) {
+    const int grid = grid_for(ctx, k_splat, kSplatBlock, ctx->h_header->total_pixels);
+    timed(ctx, CGPU_KERNEL_SPLAT, ctx->stream, [&] { k_splat<<<grid, kSplatBlock, 0, ctx->stream>>>(a); });
+    ctx->stats.kernel_launches += 1;
+}
+
 // rec (optional): the batch's rays are recorded there, for the adjoint.
-cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool splat, bool counting,
-                              const AdjRecords* rec = nullptr) {
+cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool counting, const AdjRecords* rec = nullptr) {
     RenderArgs a = make_args(ctx);
     // With per-kernel timing on, the shadow pass runs after the extend pass on
     // the same stream, so that each event pair brackets one kernel alone.
@@ -1180,11 +1186,6 @@ cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool spl
         if (b == depth) break;
         timed(ctx, CGPU_KERNEL_SHADE, s, [&] { launches += launch_shade(ctx, a, b, gsd); });
     }
-    if (splat) {
-        const int gsp = grid_for(ctx, k_splat, kSplatBlock, ctx->h_header->total_pixels);
-        timed(ctx, CGPU_KERNEL_SPLAT, s, [&] { k_splat<<<gsp, kSplatBlock, 0, s>>>(a); });
-        launches += 1;
-    }
     cudaEventDestroy(fork);
     cudaEventDestroy(join);
     ctx->stats.kernel_launches += launches;
@@ -1206,16 +1207,20 @@ cgpu_status run_batch(cgpu_ctx* ctx, int mode, int depth, uint32_t paths, bool s
             timed(ctx, CGPU_KERNEL_MEGAKERNEL, ctx->stream, [&] { k<<<g, bt, 0, ctx->stream>>>(a); });
         }
         ctx->stats.kernel_launches += 1;
-        if (splat) {
-            const int gsp = grid_for(ctx, k_splat, kSplatBlock, ctx->h_header->total_pixels);
-            timed(ctx, CGPU_KERNEL_SPLAT, ctx->stream, [&] { k_splat<<<gsp, kSplatBlock, 0, ctx->stream>>>(a); });
-            ctx->stats.kernel_launches += 1;
-        }
+        if (splat) launch_splat(ctx, a);
         return cg_cuda(ctx, cudaGetLastError(), "megakernel launch");
     }
-    if (!use_graph || counting || !splat || ctx->profiling) return enqueue_wavefront(ctx, depth, paths, splat, counting);
+    if (!use_graph || counting || !splat || ctx->profiling) {
+        const cgpu_status st = enqueue_wavefront(ctx, depth, paths, counting);
+        if (st != CGPU_OK || !splat) return st;
+        launch_splat(ctx, make_args(ctx));
+        return cg_cuda(ctx, cudaGetLastError(), "splat launch");
+    }
     // one graph per traversal variant, captured anew when the depth, the path capacity or the other
-    // kernels change; the batch itself lives in device memory
+    // kernels change; the batch itself lives in device memory.  The splat follows it: its grid goes by
+    // the batch's own pixels (with the grid of the batch that was captured first, a 24 x 20 frame, a
+    // 1280 x 720 frame of 16 samples took 59.4 ms instead of 13.5; with the grid of the path capacity, a
+    // 333 x 251 frame 1.91 instead of 1.88).
     cgpu_ctx::Graph& G = ctx->graphs[ctx->batch_closest >= 2 ? 1 : 0];
     if (!G.exec || G.depth != depth || G.paths != ctx->path_cap || G.spheres != ctx->batch_spheres ||
         G.kinds != ctx->batch_kinds) {
@@ -1228,7 +1233,7 @@ cgpu_status run_batch(cgpu_ctx* ctx, int mode, int depth, uint32_t paths, bool s
         if (e != cudaSuccess) return cg_cuda(ctx, e, "begin capture");
         const uint32_t before = ctx->stats.kernel_launches;
         // capture for the full capacity: kernels read the live path count from the header
-        cgpu_status st = enqueue_wavefront(ctx, depth, ctx->path_cap, true, false);
+        cgpu_status st = enqueue_wavefront(ctx, depth, ctx->path_cap, false);
         e = cudaStreamEndCapture(ctx->stream, &g);
         if (st != CGPU_OK) return st;
         if (e != cudaSuccess) return cg_cuda(ctx, e, "end capture");
@@ -1243,7 +1248,10 @@ cgpu_status run_batch(cgpu_ctx* ctx, int mode, int depth, uint32_t paths, bool s
         ctx->stats.kernel_launches = before;
     }
     ctx->stats.kernel_launches += G.launches;
-    return cg_cuda(ctx, cudaGraphLaunch(G.exec, ctx->stream), "graph launch");
+    const cudaError_t e = cudaGraphLaunch(G.exec, ctx->stream);
+    if (e != cudaSuccess) return cg_cuda(ctx, e, "graph launch");
+    launch_splat(ctx, make_args(ctx));
+    return cg_cuda(ctx, cudaGetLastError(), "splat launch");
 }
 
 }  // namespace
@@ -1633,7 +1641,7 @@ cgpu_status cg_adjoint_wavefront(cgpu_ctx* ctx, int scene, uint32_t spp, uint64_
         h.seed = seed;
         cudaMemcpyAsync(ctx->d_chunks, ctx->h_chunks, sizeof(Chunk), cudaMemcpyHostToDevice, ctx->stream);
         cudaMemcpyAsync(ctx->d_header, ctx->h_header, sizeof(BatchHeader), cudaMemcpyHostToDevice, ctx->stream);
-        st = enqueue_wavefront(ctx, depth, paths, false, false, &rec);
+        st = enqueue_wavefront(ctx, depth, paths, false, &rec);
         if (st != CGPU_OK) return st;
         enqueue_adjoint_replay(ctx, a, rec, depth, paths, shared_bytes);
         st = cg_cuda(ctx, cudaGetLastError(), "adjoint wavefront launch");
