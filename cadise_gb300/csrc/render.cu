@@ -396,44 +396,15 @@ __global__ void __maxnreg__(kPersistRegs) k_wf_extend_pww(RenderArgs a, int b) {
 
 constexpr int kTieBlock = 64;
 
-// The hit of a closest-hit ray that the persistent pass left with `held` and
-// another record within the tie window (`other`): held or other by closer_hit's
-// rules, other's distance worked out again by the same test.  Of several (-2) the
-// pass has only the nearest, held: the ray is traced again through the nodes
-// within the window of it, twice as wide to either side (a node that ends before
-// it, or begins behind it, holds none of them).
-template <bool COUNT, bool SPH>
-CG_D HitD tie_hit(const SceneD& S, const RayPre& r, HitD held, int other, TraceCounters* cnt) {
-    if (other < 0) {
-        const float slack = fabsf(held.t) * (kTieSlack - 1.0f) + S.tie_abs;
-        const float near = held.t - 2.0f * slack, far = held.t + 4.0f * slack;
-        if (!traverse<false, COUNT, SPH>(S, r, fmaxf(r.tmin, near), fminf(r.tmax, far), &held, cnt)) held.slot = -1;
-        return held;
-    }
-    const float4* tp = reinterpret_cast<const float4*>(S.tris + other);
-    const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
-    float t, u, v;
-    const float bound = tie_hi(S, tie_hi(S, held.t));
-    const bool sphere = SPH && (__float_as_uint(c.w) & 3u) == kRecSphere;
-    if ((sphere ? sphere_test(r, f3(a), b.x, bound, &t) : tri_test(r, f3(a), f3(b), f3(c), bound, &t, &u, &v)) &&
-        closer_hit(S, r, t, __float_as_int(a.w), other, held.t, held.slot)) {
-        held.t = t;
-        held.slot = other;
-    }
-    return held;
-}
-
 // Closest-hit rays the persistent pass left to this kernel (q_tie): two
 // primitives within the tie window of each other, which tie_prefers orders
-// by the reference's own test and tie order.  Of two the pass has both records
-// and only the comparison is left; of more the ray is traced again with the
-// per-ray traversal (closer_hit / tie_prefers), within the window of the hit.
-// Then it is finished as the persistent pass finishes its other rays.  Bound by
-// latency: few rays, and a launch that traced some of them again from their
-// origins lasted 105 us whatever their number (33 launches of a frame of 2 M
-// triangles under a sky: 3.45 ms, 1.30 within the window; 1 M triangles 0.95 and
-// 0.45).  It runs beside the any-hit pass (on the other
-// stream), and its grid strides over however few rays it got.
+// by the reference's own test and tie order (tie_hit).  Of two the pass has both
+// records and only the comparison is left; of more the ray is traced again with
+// the per-ray traversal.  Then it is finished as the persistent pass finishes its
+// other rays.  Bound by latency: few rays, and a launch that traces some of them
+// from their origins lasts about 100 us whatever their number.  It runs beside
+// the any-hit pass (on the other stream), and its grid strides over however few
+// rays it got.
 template <bool COUNT, bool SPH>
 __global__ void k_wf_ties(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;

@@ -438,14 +438,11 @@ CG_D bool visit_leaf(const SceneD& S, const RayPre& r, uint32_t e, float& tcur, 
 // megakernel's traversal (its threads are at different bounces anyway) and
 // every any-hit query (the first hit ends the walk, so there is nothing to
 // gain from holding leaves back).
-// Nodes that end before `near` are left out, and hits beyond `far`.
 template <bool ANY, bool COUNT, bool SPH = true>
-CG_D bool traverse(const SceneD& S, const RayPre& r, float near, float far, HitD* hit, TraceCounters* cnt) {
+CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* cnt) {
     LocalStack stack;
     int sp = 0;
-    RayPre box = r;
-    box.tmin = near;
-    float tcur = far;
+    float tcur = r.tmax;
     int hslot = -1;
     float hu = 0.0f, hv = 0.0f;
     uint32_t cur = 0;  // root first (always an inner node)
@@ -460,7 +457,7 @@ CG_D bool traverse(const SceneD& S, const RayPre& r, float near, float far, HitD
                 return true;
             }
         } else {
-            next = visit_node<ANY, COUNT>(S, box, cur, tcur, stack, sp, cnt);
+            next = visit_node<ANY, COUNT>(S, r, cur, tcur, stack, sp, cnt);
         }
         // else the next stack entry that can still hold a closer hit
         while (next == kNoEntry && sp > 0) {
@@ -477,9 +474,30 @@ CG_D bool traverse(const SceneD& S, const RayPre& r, float near, float far, HitD
     return hslot >= 0;
 }
 
-template <bool ANY, bool COUNT, bool SPH = true>
-CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* cnt) {
-    return traverse<ANY, COUNT, SPH>(S, r, r.tmin, r.tmax, hit, cnt);
+// The hit of a closest-hit ray that the persistent pass left with `held` and
+// another record within the tie window (`other`): held or other by closer_hit's
+// rules, other's distance worked out again by the same test.  Of several (-2) the
+// pass has only the nearest, held: the ray is traced again, from its origin.  (A
+// walk through the nodes around held's distance alone is shorter but loses hits:
+// a sliver's distance can lie outside its own box's interval.)  `held` stands
+// where the walk meets nothing.
+template <bool COUNT, bool SPH>
+CG_D HitD tie_hit(const SceneD& S, const RayPre& r, HitD held, int other, TraceCounters* cnt) {
+    if (other < 0) {
+        HitD h;
+        return traverse<false, COUNT, SPH>(S, r, &h, cnt) ? h : held;
+    }
+    const float4* tp = reinterpret_cast<const float4*>(S.tris + other);
+    const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
+    float t, u, v;
+    const float bound = tie_hi(S, tie_hi(S, held.t));
+    const bool sphere = SPH && (__float_as_uint(c.w) & 3u) == kRecSphere;
+    if ((sphere ? sphere_test(r, f3(a), b.x, bound, &t) : tri_test(r, f3(a), f3(b), f3(c), bound, &t, &u, &v)) &&
+        closer_hit(S, r, t, __float_as_int(a.w), other, held.t, held.slot)) {
+        held.t = t;
+        held.slot = other;
+    }
+    return held;
 }
 
 // Whether a primitive other than `prim_l` comes before the hit (t_l, prim_l,
