@@ -178,6 +178,11 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
     int pool = 0, pool_end = 0;
     bool drained = false;
     const int lane = threadIdx.x & 31;
+    float box_abs = 0.0f;
+    // tie_hi and box_widen; at a negative t the relative part shrinks the bound, and
+    // the absolute parts make up for it (at least as wide as theirs; tie_hit decides)
+    auto tie_widen = [&](float t) { return t * (1.0f + kTieSlack) + tie_abs; };
+    auto widen = [&](float t) { return GENERAL ? fmaf(t, 1.0f + kBoxSlack, box_abs) : t * (1.0f + kBoxSlack); };
 
     for (;;) {
         // ---- finished lanes take the next rays of the warp's share of the queue
@@ -203,7 +208,14 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                 const SceneD* S = scenes + scene;
                 nodes = S->nodes;
                 tris = S->tris;
-                if (!ANY) tie_abs = S->tie_abs;
+                if (!ANY || GENERAL) tie_abs = S->tie_abs;
+                if (GENERAL) {
+                    // no distance in the scene is below -reach
+                    const float reach = fminf(fmaxf(-ray_tmin, 0.0f),
+                                              fabsf(r.o.x) + fabsf(r.o.y) + fabsf(r.o.z) + 0x1p17f * tie_abs);
+                    box_abs = 2.0f * kBoxSlack * reach;
+                    tie_abs += 2.0f * kTieSlack * reach;
+                }
                 left = int(min(S->visit_budget, 0x7FFFFFFFu));
                 pray_prep(r, d);
                 hslot = -1;
@@ -219,7 +231,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
         // ---- steps
         for (int round = kRoundSteps - 1;;) {
             const float tmin = GENERAL ? ray_tmin : kRayEps;
-            const float tcull = GENERAL && !ANY ? tcur * kTieSlack + tie_abs : tcur;
+            const float tcull = GENERAL && !ANY ? tie_widen(tcur) : tcur;
             // a leaf is postponed (once); a lane without a node takes its next
             // stack entry (one a step: a culled one costs it the step)
             if (cur < -1 && leaf == -1) {
@@ -248,7 +260,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                     "setp.le.and.f32 q, t, %3, p;\n\t"
                     "@q mov.b32 %0, e;\n\t}"
                     : "+r"(cur), "+r"(stack.sp)
-                    : "r"(stack.base), "f"(tcull * kBoxSlack));
+                    : "r"(stack.base), "f"(widen(tcull)));
             }
             if (cur < -1 && leaf == -1) {
                 leaf = cur;
@@ -274,7 +286,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                     load_node(nodes, uint32_t(cur), nd);
                     if (COUNT) tc.nodes++;
                     float tn[4];
-                    child_hits(r.o, r.inv, tmin, nd, tcull, tn);
+                    child_hits(r.o, r.inv, tmin, nd, tcull, widen, tn);
                     const uint32_t ce[4] = {__float_as_uint(nd[1].x), __float_as_uint(nd[1].y),
                                             __float_as_uint(nd[1].z), __float_as_uint(nd[1].w)};
                     // room for the three children a visit may push
@@ -336,7 +348,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                 const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
                 if (COUNT) tc.tris++;
                 leaf = (leaf & 0x70000000) ? leaf - 0x10000000 + 1 : -1;
-                const float bound = ANY ? tcur : tcur * kTieSlack + tie_abs;
+                const float bound = ANY ? tcur : tie_widen(tcur);
                 float t;
                 bool hit;
                 bool sphere = false;
@@ -361,7 +373,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                         const int held = hslot & kSlotMask;
                         const bool nearer = first ? t <= tcur : (t < tcur || (t == tcur && int(slot) < held));
                         // a hit nearer by more than the window clears what the held one was tied with
-                        const bool tied = !first && t * kTieSlack + tie_abs >= tcur;
+                        const bool tied = !first && tie_widen(t) >= tcur;
                         if (tied) other = other == -1 ? (nearer ? held : int(slot)) : -2;
                         else if (nearer) other = -1;
                         if (nearer) {

@@ -808,15 +808,23 @@ __global__ void k_trace(const SceneD* scenes, int scene, const cgpu_ray* rays, u
         const SceneD& S = scenes[scene];
         const cgpu_ray r = rays[i];
         // the direction is normalised again, as the reference's Ray constructor does (ray.cpp:19-30)
-        const RayPre pr = ray_prep(mk(r.org[0], r.org[1], r.org[2]), normalize(mk(r.dir[0], r.dir[1], r.dir[2])),
-                                   r.t_min, r.t_max);
-        HitD h;
-        TraceCounters tc{0, 0};
-        if (occ) {
-            occ[i] = traverse<true, false>(S, pr, &h, &tc) ? 1 : 0;
+        RayPre pr = ray_prep(mk(r.org[0], r.org[1], r.org[2]), normalize(mk(r.dir[0], r.dir[1], r.dir[2])), r.t_min, r.t_max);
+        auto answer = [&](const RayPre& p) {
+            HitD h;
+            TraceCounters tc{0, 0};
+            if (occ) {
+                occ[i] = traverse<true, false>(S, p, &h, &tc) ? 1 : 0;
+            } else {
+                if (!traverse_warp<false>(S, p, &h, &tc)) h.slot = -1;
+                hits[i] = query_answer(S, p.o, p.d, h);
+            }
+        };
+        // the mask a constant where it can be (one form for all costs 257 rays 2 %)
+        if (r.t_min < 0.0f) {
+            answer(pr);
         } else {
-            if (!traverse_warp<false>(S, pr, &h, &tc)) h.slot = -1;
-            hits[i] = query_answer(S, pr.o, pr.d, h);
+            pr.mag = 0xFFFFFFFFu;
+            answer(pr);
         }
     }
 }

@@ -13,8 +13,8 @@
 // primitives met within a few roundings of each other (a ray through an edge
 // two triangles share, coplanar overlapping quads) are ordered by the
 // reference's own test and tie order (tie_prefers), so the closest hit is the
-// reference's there too.  Box tests widen t_max by 1 + 2 gamma(3) (and by the
-// tie window for closest hits) to stay conservative.
+// reference's there too.  Box tests widen t_max by 10 x 2^-24 of itself (and by
+// the tie window for closest hits) to stay conservative.
 #pragma once
 
 #include "scene_device.cuh"
@@ -26,6 +26,7 @@ struct RayPre {
     float tmin, tmax;
     int kx, ky, kz;
     float Sx, Sy, Sz;
+    uint32_t mag;  // mask of the bits of |t|, all ones where t is never negative (a render: a constant)
 };
 
 CG_D RayPre ray_prep(float3 o, float3 d, float tmin, float tmax) {
@@ -34,6 +35,7 @@ CG_D RayPre ray_prep(float3 o, float3 d, float tmin, float tmax) {
     r.d = d;
     r.tmin = tmin;
     r.tmax = tmax;
+    r.mag = tmin < 0.0f ? 0x7FFFFFFFu : 0xFFFFFFFFu;
     // zero components would make (lo - o) * inf = NaN on a box face plane
     const float e = 1e-30f;
     const float dx = fabsf(d.x) < e ? copysignf(e, d.x) : d.x;
@@ -158,23 +160,28 @@ CG_D void load_node(const Bvh4Node* nodes, uint32_t idx, float4 (&q)[4]) {
 
 // Closest-hit tie window (tie_prefers): candidates whose distances lie within
 // tie_hi of each other are ordered by the reference's rule, so closest-hit
-// bounds are widened to tie_hi, and box distances by a further 1 + 2 gamma(3).
+// bounds are widened to tie_hi, and box distances further (box_widen).
 // The window is relative (kTieSlack) plus absolute (SceneD::tie_abs, 2^-16 of
 // the scene's coordinate scale): the watertight distance of a short ray
 // carries the rounding of vertex coordinates of the scene's magnitude, up to
 // 3e-6 of the scale on the reference's test scenes.
-constexpr float kTieSlack = 1.000004f;
-CG_D float tie_hi(const SceneD& S, float t) { return t * kTieSlack + S.tie_abs; }
+// The relative part is of |t|: a query's distances may be negative.
+constexpr float kTieSlack = 34 * 0x1p-23f;  // 4.05e-6
+CG_D float widen(const RayPre& r, float t, float slack) { return fmaf(__uint_as_float(__float_as_uint(t) & r.mag), slack, t); }
+CG_D float tie_hi(const SceneD& S, const RayPre& r, float t) { return widen(r, t, kTieSlack) + S.tie_abs; }
 
-// Box tests widen by 1 + 10 x 2^-24: three roundings of each plane's distance,
-// and one more each for a reciprocal unit's 1 / d.
-constexpr float kBoxSlack = 1.0000006f;
+// Box tests widen by 10 x 2^-24 of the distance: three roundings of each plane's
+// distance, and one more each for a reciprocal unit's 1 / d.
+constexpr float kBoxSlack = 5 * 0x1p-23f;
+CG_D float box_widen(const RayPre& r, float t) { return widen(r, t, kBoxSlack); }
 
 // Child box distances; tnear = +inf marks a miss.  Empty child slots hold
 // entry 0 (the root, never anyone's child) and are always a miss.  Per axis
 // the slab distances are a + q * b with a = (origin - o) / d and b = step / d
 // (exact: the step is a power of two), the near plane picked by the sign of d.
-CG_D void child_hits(float3 o, float3 inv, float tmin, const float4 (&q)[4], float tcur, float (&tn)[4]) {
+// `widen` is the conservative bound of a distance (box_widen).
+template <class Widen>
+CG_D void child_hits(float3 o, float3 inv, float tmin, const float4 (&q)[4], float tcur, Widen&& widen, float (&tn)[4]) {
     const uint32_t ce[4] = {__float_as_uint(q[1].x), __float_as_uint(q[1].y), __float_as_uint(q[1].z),
                             __float_as_uint(q[1].w)};
     const uint32_t exps = __float_as_uint(q[0].w);
@@ -192,7 +199,7 @@ CG_D void child_hits(float3 o, float3 inv, float tmin, const float4 (&q)[4], flo
     const uint32_t nx = sx ? hix : lox, fx = sx ? lox : hix;
     const uint32_t ny = sy ? hiy : loy, fy = sy ? loy : hiy;
     const uint32_t nz = sz ? hiz : loz, fz = sz ? loz : hiz;
-    const float tlim = tcur * kBoxSlack;
+    const float tlim = widen(tcur);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int sh = 8 * i;
@@ -202,7 +209,7 @@ CG_D void child_hits(float3 o, float3 inv, float tmin, const float4 (&q)[4], flo
         const float tnear = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, tmin));
         const float tfar = fminf(fminf(tfx, tfy), fminf(tfz, tlim));
         // slot 0 is never empty
-        tn[i] = ((i == 0 || ce[i] != 0u) && tnear <= tfar * kBoxSlack) ? tnear : __int_as_float(0x7f800000);
+        tn[i] = ((i == 0 || ce[i] != 0u) && tnear <= widen(tfar)) ? tnear : __int_as_float(0x7f800000);
     }
 }
 
@@ -247,7 +254,7 @@ CG_D uint32_t visit_node(const SceneD& S, const RayPre& r, uint32_t e, float tcu
     load_node(S.nodes, e, q);
     if (COUNT) cnt->nodes++;
     float tn[4];
-    child_hits(r.o, r.inv, r.tmin, q, ANY ? tcur : tie_hi(S, tcur), tn);
+    child_hits(r.o, r.inv, r.tmin, q, ANY ? tcur : tie_hi(S, r, tcur), [&](float t) { return box_widen(r, t); }, tn);
     uint32_t ce[4] = {__float_as_uint(q[1].x), __float_as_uint(q[1].y), __float_as_uint(q[1].z),
                       __float_as_uint(q[1].w)};
     if (!ANY) {
@@ -391,8 +398,8 @@ CG_D bool tie_prefers(const SceneD& S, const RayPre& r, int slot, int prim, floa
 // candidate's; the kept hit's primitive is loaded only inside the window.
 CG_D bool closer_hit(const SceneD& S, const RayPre& r, float t, int prim, int slot, float tcur, int hslot) {
     if (hslot < 0) return t <= tcur;
-    if (tie_hi(S, t) < tcur) return true;
-    if (t > tie_hi(S, tcur)) return false;
+    if (tie_hi(S, r, t) < tcur) return true;
+    if (t > tie_hi(S, r, tcur)) return false;
     const int kept = __float_as_int(ldg4(reinterpret_cast<const float4*>(S.tris + hslot)).w);
     if (prim == kept) return t < tcur || (t == tcur && slot < hslot);
     return tie_prefers(S, r, slot, prim, t, hslot, kept, tcur);
@@ -415,7 +422,7 @@ CG_D bool visit_leaf(const SceneD& S, const RayPre& r, uint32_t e, float& tcur, 
         // closest hit: a bound as wide as the tie window, so that every
         // primitive within it reaches closer_hit
         const bool sphere = SPH && (__float_as_uint(c.w) & 3u) == kRecSphere;
-        const float bound = ANY ? tcur : tie_hi(S, tcur);
+        const float bound = ANY ? tcur : tie_hi(S, r, tcur);
         if (sphere ? sphere_test(r, f3(a), b.x, bound, &t) : tri_test(r, f3(a), f3(b), f3(c), bound, &t, &u, &v)) {
             const int slot = int(first + k);
             if (ANY) {
@@ -462,7 +469,7 @@ CG_D bool traverse(const SceneD& S, const RayPre& r, HitD* hit, TraceCounters* c
         // else the next stack entry that can still hold a closer hit
         while (next == kNoEntry && sp > 0) {
             --sp;
-            if (ANY || stack.dist(sp) <= tie_hi(S, tcur) * kBoxSlack) next = stack.entry(sp);
+            if (ANY || stack.dist(sp) <= box_widen(r, tie_hi(S, r, tcur))) next = stack.entry(sp);
         }
         if (next == kNoEntry) break;
         cur = next;
@@ -490,7 +497,7 @@ CG_D HitD tie_hit(const SceneD& S, const RayPre& r, HitD held, int other, TraceC
     const float4* tp = reinterpret_cast<const float4*>(S.tris + other);
     const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
     float t, u, v;
-    const float bound = tie_hi(S, tie_hi(S, held.t));
+    const float bound = tie_hi(S, r, tie_hi(S, r, held.t));
     const bool sphere = SPH && (__float_as_uint(c.w) & 3u) == kRecSphere;
     if ((sphere ? sphere_test(r, f3(a), b.x, bound, &t) : tri_test(r, f3(a), f3(b), f3(c), bound, &t, &u, &v)) &&
         closer_hit(S, r, t, __float_as_int(a.w), other, held.t, held.slot)) {
@@ -511,7 +518,7 @@ template <bool COUNT, bool SPH = true>
 CG_D bool visit_leaf_before(const SceneD& S, const RayPre& r, uint32_t e, float t_l, int prim_l, int slot_l,
                             TraceCounters* cnt) {
     const uint32_t first = leaf_first(e), n = leaf_count(e);
-    const float bound = tie_hi(S, t_l);
+    const float bound = tie_hi(S, r, t_l);
     for (uint32_t k = 0; k < n; ++k) {
         const float4* tp = reinterpret_cast<const float4*>(S.tris + first + k);
         const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
@@ -525,7 +532,7 @@ CG_D bool visit_leaf_before(const SceneD& S, const RayPre& r, uint32_t e, float 
                 if (t <= t_l) return true;
                 continue;
             }
-            if (tie_hi(S, t) < t_l) return true;
+            if (tie_hi(S, r, t) < t_l) return true;
             if (tie_prefers(S, r, int(first + k), prim, t, slot_l, prim_l, t_l)) return true;
         }
     }
@@ -538,7 +545,7 @@ CG_D bool occluded_before(const SceneD& S, const RayPre& r, float t_l, int prim_
     int sp = 0;
     uint32_t cur = 0;
     uint32_t left = S.visit_budget;
-    const float tb = tie_hi(S, t_l);
+    const float tb = tie_hi(S, r, t_l);
     for (;;) {
         if (over_budget(S, left)) return false;
         uint32_t next = kNoEntry;
@@ -575,7 +582,7 @@ CG_D bool traverse_warp(const SceneD& S, const RayPre& r, HitD* hit, TraceCounte
     auto pop = [&]() -> uint32_t {
         while (sp > 0) {
             --sp;
-            if (stack.dist(sp) <= tie_hi(S, tcur) * kBoxSlack) return stack.entry(sp);
+            if (stack.dist(sp) <= box_widen(r, tie_hi(S, r, tcur))) return stack.entry(sp);
         }
         return kNoEntry;
     };
@@ -665,7 +672,7 @@ CG_D void trav_step(const SceneD& S, const RayPre& r, TravState& st, TraceCounte
     }
     while (st.sp > 0) {
         --st.sp;
-        if (ANY || st.stack.dist(st.sp) <= tie_hi(S, st.tcur) * kBoxSlack) {
+        if (ANY || st.stack.dist(st.sp) <= box_widen(r, tie_hi(S, r, st.tcur))) {
             st.cur = st.stack.entry(st.sp);
             return;
         }

@@ -1,8 +1,10 @@
-// CPU execution of what follows the persistent passes' closest hits (tie_hit;
-// test infrastructure, never part of the library).
+// CPU execution of what follows the persistent passes' closest hits (tie_hit)
+// and of queries against every record of a scene (test infrastructure, never
+// part of the library).
 #include "../../cadise_gb300/csrc/scene_build.h"
 #include "../../cadise_gb300/csrc/traverse.cuh"
 
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <memory>
@@ -67,9 +69,35 @@ void tc_several(void* p, const float* rays, uint32_t n, int32_t* held, int32_t* 
         if (h.slot < 0) continue;
         for (size_t k = 0; k < sc.hs.tris.size(); ++k) {
             float t;
-            held[2 * i + 1] += record_hit(S, r, k, cg::tie_hi(S, h.t), &t);
+            held[2 * i + 1] += record_hit(S, r, k, cg::tie_hi(S, r, h.t), &t);
         }
         resolved[i] = cg::tie_hit<false, true>(S, r, h, -2, &tc).slot;
+    }
+}
+
+// Per ray (8 floats): t[3 i] the smallest distance of all records, t[3 i + 1] that
+// of the traversal, t[3 i + 2] that of the warp traversal (3.4e38: a miss);
+// any[i] the any-hit traversal's answer; window[i] how far two distances may lie
+// apart and still be ordered by the reference's rule.
+void tc_closest(void* p, const float* rays, uint32_t n, float* t, int32_t* any, float* window) {
+    const Scene& sc = *static_cast<Scene*>(p);
+    const cg::SceneD& S = sc.S;
+    for (uint32_t i = 0; i < n; ++i) {
+        const cg::RayPre r = prep(rays + 8 * size_t(i));
+        float best = r.tmax, tk;
+        bool found = false;
+        for (size_t k = 0; k < sc.hs.tris.size(); ++k)
+            if (record_hit(S, r, k, best, &tk) && tk <= best) {
+                best = tk;
+                found = true;
+            }
+        cg::TraceCounters tc{0, 0};
+        cg::HitD a, b, c;
+        t[3 * i] = found ? best : 3.4e38f;
+        t[3 * i + 1] = cg::traverse<false, false>(S, r, &a, &tc) ? a.t : 3.4e38f;
+        t[3 * i + 2] = cg::traverse_warp<false>(S, r, &b, &tc) ? b.t : 3.4e38f;
+        any[i] = cg::traverse<true, false>(S, r, &c, &tc);
+        window[i] = std::fabs(cg::tie_hi(S, r, best) - best);
     }
 }
 
