@@ -152,12 +152,15 @@ CG_D void pray_prep(PRay<SPH>& r, float3 d) {
 // loads entry k and returns the caller's id of the ray; finish(done, id, t,
 // slot, kind, other) is called by the whole warp with the lanes whose ray is done
 // (slot < 0: a miss; kind: the record's shade queue; other: the record that met
-// the ray within the tie window of slot, -1 none, -2 more than one);
+// the ray within the tie reach of slot, -1 none, -2 more than one);
 // exhausted(id): the ray ran out of its visit budget.
-// GENERAL (ray queries): every ray has its own tmin, and closest-hit rays cull
-// nodes by the tie window's far end, so that every primitive within the window
-// is met; the render's rays all start at kRayEps and cull by the hit itself
-// (4 % faster; ties are then found where both primitives are met).
+// The tie reach of a hit is three tie windows wide, and closest-hit rays cull by
+// its far end, so that every record within it is met, whatever the order of the
+// visits.  Two windows hold all records that tie with the hit or with one that
+// ties with it: of a hit and a single other in its reach the two alone decide
+// (tie_hit).  The third stands in for box_widen.
+// GENERAL (ray queries): every ray has its own tmin, which may be negative; the
+// render's rays all start at kRayEps.
 template <bool ANY, bool COUNT, bool SPH, bool GENERAL, class Fetch, class Finish, class Exhausted>
 CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fetch&& fetch, Finish&& finish,
                           Exhausted&& exhausted, TraceCounters& tc) {
@@ -167,10 +170,10 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
     PRay<SPH> r{};
     const Bvh4Node* nodes = nullptr;
     const TriRecord* tris = nullptr;
-    float tie_abs = 0.0f;
+    float tie_abs = 0.0f;  // the absolute part of the tie reach
     float tcur = 0.0f, ray_tmin = 0.0f;
     int hslot = -1;
-    int other = -1;      // the record within the tie window of hslot: -1 none, -2 more than one
+    int other = -1;      // the record within the tie reach of hslot: -1 none, -2 more than one
     int left = 0;        // node and leaf visits left, negative once the budget is exceeded
     int cur = -1;        // next entry: an inner node (>= 0), a leaf (< -1), -1 none
     int leaf = -1;       // postponed leaf, -1 none
@@ -179,9 +182,9 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
     bool drained = false;
     const int lane = threadIdx.x & 31;
     float box_abs = 0.0f;
-    // tie_hi and box_widen; at a negative t the relative part shrinks the bound, and
-    // the absolute parts make up for it (at least as wide as theirs; tie_hit decides)
-    auto tie_widen = [&](float t) { return t * (1.0f + kTieSlack) + tie_abs; };
+    // the far end of the tie reach, and box_widen: at a negative t the relative part
+    // shrinks the bound, and the absolute parts make up for it
+    auto reach = [&](float t) { return fmaf(t, 1.0f + 3.0f * kTieSlack, tie_abs); };
     auto widen = [&](float t) { return GENERAL ? fmaf(t, 1.0f + kBoxSlack, box_abs) : t * (1.0f + kBoxSlack); };
 
     for (;;) {
@@ -208,13 +211,13 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                 const SceneD* S = scenes + scene;
                 nodes = S->nodes;
                 tris = S->tris;
-                if (!ANY || GENERAL) tie_abs = S->tie_abs;
+                if (!ANY) tie_abs = 3.0f * S->tie_abs;
                 if (GENERAL) {
-                    // no distance in the scene is below -reach
-                    const float reach = fminf(fmaxf(-ray_tmin, 0.0f),
-                                              fabsf(r.o.x) + fabsf(r.o.y) + fabsf(r.o.z) + 0x1p17f * tie_abs);
-                    box_abs = 2.0f * kBoxSlack * reach;
-                    tie_abs += 2.0f * kTieSlack * reach;
+                    // no distance in the scene is below -far
+                    const float far = fminf(fmaxf(-ray_tmin, 0.0f),
+                                            fabsf(r.o.x) + fabsf(r.o.y) + fabsf(r.o.z) + 0x1p17f * S->tie_abs);
+                    box_abs = 2.0f * kBoxSlack * far;
+                    if (!ANY) tie_abs += 6.0f * kTieSlack * far;
                 }
                 left = int(min(S->visit_budget, 0x7FFFFFFFu));
                 pray_prep(r, d);
@@ -231,7 +234,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
         // ---- steps
         for (int round = kRoundSteps - 1;;) {
             const float tmin = GENERAL ? ray_tmin : kRayEps;
-            const float tcull = GENERAL && !ANY ? tie_widen(tcur) : tcur;
+            const float tlim = ANY ? widen(tcur) : reach(tcur);
             // a leaf is postponed (once); a lane without a node takes its next
             // stack entry (one a step: a culled one costs it the step)
             if (cur < -1 && leaf == -1) {
@@ -260,7 +263,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                     "setp.le.and.f32 q, t, %3, p;\n\t"
                     "@q mov.b32 %0, e;\n\t}"
                     : "+r"(cur), "+r"(stack.sp)
-                    : "r"(stack.base), "f"(widen(tcull)));
+                    : "r"(stack.base), "f"(tlim));
             }
             if (cur < -1 && leaf == -1) {
                 leaf = cur;
@@ -286,7 +289,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                     load_node(nodes, uint32_t(cur), nd);
                     if (COUNT) tc.nodes++;
                     float tn[4];
-                    child_hits(r.o, r.inv, tmin, nd, tcull, widen, tn);
+                    child_hits(r.o, r.inv, tmin, nd, tlim, widen, tn);
                     const uint32_t ce[4] = {__float_as_uint(nd[1].x), __float_as_uint(nd[1].y),
                                             __float_as_uint(nd[1].z), __float_as_uint(nd[1].w)};
                     // room for the three children a visit may push
@@ -348,7 +351,7 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                 const float4 a = ldg4(tp), b = ldg4(tp + 1), c = ldg4(tp + 2);
                 if (COUNT) tc.tris++;
                 leaf = (leaf & 0x70000000) ? leaf - 0x10000000 + 1 : -1;
-                const float bound = ANY ? tcur : tie_widen(tcur);
+                const float bound = ANY ? tcur : tlim;
                 float t;
                 bool hit;
                 bool sphere = false;
@@ -372,8 +375,8 @@ CG_D void persistent_pass(const SceneD* scenes, int* work, int n, int refill, Fe
                         const bool first = hslot < 0;
                         const int held = hslot & kSlotMask;
                         const bool nearer = first ? t <= tcur : (t < tcur || (t == tcur && int(slot) < held));
-                        // a hit nearer by more than the window clears what the held one was tied with
-                        const bool tied = !first && tie_widen(t) >= tcur;
+                        // a hit nearer by more than the reach clears what the held one was tied with
+                        const bool tied = !first && reach(t) >= tcur;
                         if (tied) other = other == -1 ? (nearer ? held : int(slot)) : -2;
                         else if (nearer) other = -1;
                         if (nearer) {

@@ -179,9 +179,10 @@ CG_D float box_widen(const RayPre& r, float t) { return widen(r, t, kBoxSlack); 
 // entry 0 (the root, never anyone's child) and are always a miss.  Per axis
 // the slab distances are a + q * b with a = (origin - o) / d and b = step / d
 // (exact: the step is a power of two), the near plane picked by the sign of d.
-// `widen` is the conservative bound of a distance (box_widen).
+// `tlim`: the conservative bound of the distances that still matter; `widen` that
+// of any distance (box_widen).
 template <class Widen>
-CG_D void child_hits(float3 o, float3 inv, float tmin, const float4 (&q)[4], float tcur, Widen&& widen, float (&tn)[4]) {
+CG_D void child_hits(float3 o, float3 inv, float tmin, const float4 (&q)[4], float tlim, Widen&& widen, float (&tn)[4]) {
     const uint32_t ce[4] = {__float_as_uint(q[1].x), __float_as_uint(q[1].y), __float_as_uint(q[1].z),
                             __float_as_uint(q[1].w)};
     const uint32_t exps = __float_as_uint(q[0].w);
@@ -199,7 +200,6 @@ CG_D void child_hits(float3 o, float3 inv, float tmin, const float4 (&q)[4], flo
     const uint32_t nx = sx ? hix : lox, fx = sx ? lox : hix;
     const uint32_t ny = sy ? hiy : loy, fy = sy ? loy : hiy;
     const uint32_t nz = sz ? hiz : loz, fz = sz ? loz : hiz;
-    const float tlim = widen(tcur);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int sh = 8 * i;
@@ -254,7 +254,8 @@ CG_D uint32_t visit_node(const SceneD& S, const RayPre& r, uint32_t e, float tcu
     load_node(S.nodes, e, q);
     if (COUNT) cnt->nodes++;
     float tn[4];
-    child_hits(r.o, r.inv, r.tmin, q, ANY ? tcur : tie_hi(S, r, tcur), [&](float t) { return box_widen(r, t); }, tn);
+    child_hits(r.o, r.inv, r.tmin, q, box_widen(r, ANY ? tcur : tie_hi(S, r, tcur)),
+               [&](float t) { return box_widen(r, t); }, tn);
     uint32_t ce[4] = {__float_as_uint(q[1].x), __float_as_uint(q[1].y), __float_as_uint(q[1].z),
                       __float_as_uint(q[1].w)};
     if (!ANY) {
