@@ -15,7 +15,7 @@ namespace {
 
 bool valid_tuning(const cgpu_tuning& t) {
     auto ok_block = [](int b) { return b >= 32 && b <= 1024 && b % 32 == 0; };
-    return ok_block(t.block_trace) && ok_block(t.block_shade) && (t.traversal >= 0 && t.traversal <= 3) &&
+    return ok_block(t.block_trace) && ok_block(t.block_shade) && (t.traversal >= 0 && t.traversal <= cg::kTraversalPerRay) &&
            (t.reorder >= 0 && t.reorder <= 4) && (t.refill_closest >= 0 && t.refill_closest <= 32) &&
            (t.refill_any >= 0 && t.refill_any <= 32);
 }
@@ -39,8 +39,9 @@ std::string cache_key(cgpu_ctx* ctx, const int32_t* scenes, uint32_t n, uint32_t
         depth = std::max(depth, sl.max_depth);
     }
     std::ostringstream os;
+    // (the last field: what the values of `traversal` mean, and the search)
     os << prop.name << "|sm" << prop.multiProcessorCount << "|tris" << tris << "|pix" << pix << "|depth" << depth
-       << "|scenes" << n << "|samples" << samples;
+       << "|scenes" << n << "|samples" << samples << "|search2";
     return os.str();
 }
 
@@ -100,7 +101,7 @@ cgpu_status cgpu_tuning_set(cgpu_ctx* ctx, const cgpu_tuning* t) {
     if (!ctx || !t) return CGPU_ERR_INVALID_ARGUMENT;
     if (!valid_tuning(*t))
         return cg_fail(ctx, CGPU_ERR_INVALID_ARGUMENT,
-                       "tuning: block sizes must be multiples of 32 in [32, 1024], traversal 0 to 3, reorder 0 to 4, "
+                       "tuning: block sizes must be multiples of 32 in [32, 1024], traversal 0 to 4, reorder 0 to 4, "
                        "refill thresholds 0 to 32");
     cudaStreamSynchronize(ctx->stream);
     apply(ctx, *t);
@@ -163,6 +164,9 @@ cgpu_status cgpu_autotune(cgpu_ctx* ctx, const int32_t* scenes, uint32_t n, uint
     };
     float best_ms = 0.0f;
     cgpu_status st = time_one(best, &best_ms);
+    int closest = ctx->batch_closest, any = ctx->batch_any;  // the kernels that `best` takes
+    // every variant by its own number: where `best` leaves the choice open, the one it took is timed already
+    const int traversals[] = {1, 2, 3, cg::kTraversalPerRay};
     const int blocks[] = {64, 128, 256};
     // paths in flight: larger batches hold several samples per pixel and
     // share one tail of short late-bounce queues among them
@@ -172,28 +176,24 @@ cgpu_status cgpu_autotune(cgpu_ctx* ctx, const int32_t* scenes, uint32_t n, uint
     // queue compaction of the persistent passes: refill a warp's finished
     // lanes once fewer than this many lanes still trace
     const int refills[] = {8, 16, 24, 28, 32};
-    const int options[] = {4, 3, 3, 5, 5, 5};
-    for (int pass = 0; pass < 6 && st == CGPU_OK; ++pass) {
-        // the thresholds only act in the persistent while-while passes
-        if (pass == 4 && best.traversal < 2) continue;
-        if (pass == 5 && best.traversal < 3) continue;
+    const int options[cg::TUNE_PASSES] = {4, 3, 3, 5, 5, 5};
+    for (int pass = 0; pass < cg::TUNE_PASSES && st == CGPU_OK; ++pass) {
         for (int k = 0; k < options[pass] && st == CGPU_OK; ++k) {
             cgpu_tuning t = best;
-            if (pass == 0) t.traversal = k;
-            if (pass == 1) t.block_trace = blocks[k];
-            if (pass == 2) t.block_shade = blocks[k];
-            if (pass == 3) t.max_paths = caps[k];
-            if (pass == 4) t.refill_closest = refills[k];
-            if (pass == 5) t.refill_any = refills[k];
-            if (cg::refill_lanes(t.refill_closest) == cg::refill_lanes(best.refill_closest) &&
-                cg::refill_lanes(t.refill_any) == cg::refill_lanes(best.refill_any) && pass >= 4)
-                continue;
-            if (std::memcmp(&t, &best, sizeof(t)) == 0) continue;
+            if (pass == cg::TUNE_TRAVERSAL) t.traversal = traversals[k];
+            if (pass == cg::TUNE_BLOCK_TRACE) t.block_trace = blocks[k];
+            if (pass == cg::TUNE_BLOCK_SHADE) t.block_shade = blocks[k];
+            if (pass == cg::TUNE_MAX_PATHS) t.max_paths = caps[k];
+            if (pass == cg::TUNE_REFILL_CLOSEST) t.refill_closest = refills[k];
+            if (pass == cg::TUNE_REFILL_ANY) t.refill_any = refills[k];
+            if (cg::autotune_skips(pass, t, best, closest, any)) continue;
             float ms = 0.0f;
             st = time_one(t, &ms);
             if (st == CGPU_OK && ms < best_ms) {
                 best_ms = ms;
                 best = t;
+                closest = ctx->batch_closest;
+                any = ctx->batch_any;
             }
         }
     }

@@ -218,9 +218,31 @@ struct RenderArgs {
 constexpr int kSmallScene = 2048;
 constexpr uint64_t kLargeBatch = 1u << 19;
 
+// The kernels of a traversal variant (cgpu_tuning::traversal): 0 one ray per
+// thread, 1 persistent with ray replacement, 2 / 3 the persistent passes.
+// `persistent`: what the library would choose where the tuning leaves it open.
+constexpr int kTraversalOpen = 0, kTraversalPerRay = 4;
+inline int traversal_kernels(int traversal, bool persistent) {
+    return traversal == kTraversalPerRay ? 0 : traversal == kTraversalOpen && persistent ? 3 : traversal;
+}
+
 // The refill thresholds of a tuning, 0 replaced by the default.
 constexpr int kDefaultRefillLanes = 24;
 inline int refill_lanes(int32_t v) { return v > 0 ? v : kDefaultRefillLanes; }
+
+// cgpu_autotune's search: whether it leaves candidate `t` of a pass out, because
+// it runs the launches of `best`, which took the kernels `closest` and `any`.
+enum { TUNE_TRAVERSAL, TUNE_BLOCK_TRACE, TUNE_BLOCK_SHADE, TUNE_MAX_PATHS, TUNE_REFILL_CLOSEST, TUNE_REFILL_ANY, TUNE_PASSES };
+inline bool autotune_skips(int pass, const cgpu_tuning& t, const cgpu_tuning& best, int closest, int any) {
+    switch (pass) {
+        case TUNE_TRAVERSAL: return traversal_kernels(t.traversal, false) == closest && closest == any;
+        case TUNE_BLOCK_TRACE: return t.block_trace == best.block_trace;
+        case TUNE_BLOCK_SHADE: return t.block_shade == best.block_shade;
+        case TUNE_MAX_PATHS: return t.max_paths == best.max_paths;
+        case TUNE_REFILL_CLOSEST: return closest < 2 || refill_lanes(t.refill_closest) == refill_lanes(best.refill_closest);
+        default: return any < 3 || refill_lanes(t.refill_any) == refill_lanes(best.refill_any);
+    }
+}
 
 // Buffers of the ray reordering: keys / values ping-pong for 2 * path_cap
 // queue entries, digit counts, scan scratch, the entry count.

@@ -1043,9 +1043,8 @@ void collect_profile(cgpu_ctx* ctx) {
 // then keep one ray per thread, whose node visits do not depend on which rays
 // happen to share a warp.
 void choose_traversal(cgpu_ctx* ctx, bool closest, bool any) {
-    const int t = ctx->tuning.traversal;
-    ctx->batch_closest = t == 0 && closest && !ctx->counting ? 3 : t;
-    ctx->batch_any = t == 0 && any && !ctx->counting ? 3 : t;
+    ctx->batch_closest = traversal_kernels(ctx->tuning.traversal, closest && !ctx->counting);
+    ctx->batch_any = traversal_kernels(ctx->tuning.traversal, any && !ctx->counting);
 }
 bool large_batch(const cgpu_ctx* ctx, uint64_t paths) { return std::min<uint64_t>(paths, ctx->path_cap) >= kLargeBatch; }
 

@@ -392,25 +392,27 @@ typedef struct cgpu_tuning {
                               votes between node and triangle steps and refills a warp's finished lanes
                               once fewer than refill_closest of its lanes still trace, any-hit with one
                               ray per thread; 3: 2 plus the same persistent form for the any-hit pass
-                              (refill_any) */
+                              (refill_any); 4: one ray per thread, whatever the scene and batch */
     int32_t reorder;       /* 1, 2, 3: before each closest-hit pass after the first, sort its rays by
                               direction octant and origin (Morton order of 9, 7 or 4 bits per axis in the
                               scene bounds; 4, 3 or 2 radix passes), so that a warp traces neighbouring
-                              rays (traversal 0, 2 and 3); 4: by direction octant alone (one radix pass);
+                              rays (all but traversal 1); 4: by direction octant alone (one radix pass);
                               0: queue order (default; cgpu_autotune does not search it: on the
                               1 M-triangle field the sort costs about what it saves) */
-    int32_t refill_closest;/* queue compaction of the persistent closest-hit pass (traversal 2 and 3):
+    int32_t refill_closest;/* queue compaction of the persistent closest-hit pass (traversal 2 and 3, and
+                              0 where it takes them):
                               after each round of leaves a warp whose unfinished rays number fewer than
                               this stores its finished lanes' hits and takes the next rays of the queue
                               for them; 1..32, 0 = 24 */
-    int32_t refill_any;    /* the same threshold for the persistent any-hit pass (traversal 3); 0 = 24 */
+    int32_t refill_any;    /* the same threshold for the persistent any-hit pass (traversal 3, and 0); 0 = 24 */
 } cgpu_tuning;
 cgpu_status cgpu_tuning_get(cgpu_ctx* ctx, cgpu_tuning* out_tuning);
 cgpu_status cgpu_tuning_set(cgpu_ctx* ctx, const cgpu_tuning* tuning);
 /* Times wavefront passes of `scenes` (`samples` samples each) over a small
  * search of cgpu_tuning values (traversal variant, block sizes, the refill
  * thresholds of the persistent passes, 2^20..2^24 paths in flight) and
- * applies the fastest.  With a cache path, a result
+ * applies the fastest (traversal 0 where that stands for the fastest variant
+ * already).  With a cache path, a result
  * stored for the same GPU, scene sizes and sample count is reused without
  * timing and new results are appended (one JSON object per line). */
 cgpu_status cgpu_autotune(cgpu_ctx* ctx, const int32_t* scenes, uint32_t num_scenes, uint32_t samples,
