@@ -84,6 +84,17 @@ def traversal_profile():
         return None
 
 
+def timed_variant(tuning, kernel_times):
+    """The kernel of the timed closest-hit passes, and the tuning whose counting
+    render visits nodes as they do.  Traversal 0 leaves the variant to the
+    library, and while counting that is one ray per thread: where the timed
+    passes left rays to the tie kernel they were the persistent ones (3)."""
+    t = dict(tuning)
+    if t["traversal"] == 0 and kernel_times["ties"][1] > 0:
+        t["traversal"] = 3
+    return {1: "k_wf_extend_dyn", 2: "k_wf_extend_pww", 3: "k_wf_extend_pww"}.get(t["traversal"], "k_wf_extend"), t
+
+
 # ------------------------------------------------------------------ clocks --
 class ClockSampler:
     """nvidia-smi clock / throttle samples during the timed region (read only)."""
@@ -254,11 +265,7 @@ def run_gpu(args, rank, world, local):
         torch.cuda.synchronize()
         mk_value = float(npix) * spp * mk_steps / (e0.elapsed_time(e1) / 1e3)
 
-        # counting replay (same seeds, counters on) and per-kernel event timing
-        ctx.set_counting(True)
-        ctx.render([sid], first, 1, seed=2024, mode=cg.CGPU_MODE_WAVEFRONT, graph=False, sync=True)
-        st = ctx.stats()
-        ctx.set_counting(False)
+        # per-kernel event timing
         ctx.set_profiling(True)
         ctx.render([sid], first, 1, seed=2024, mode=cg.CGPU_MODE_WAVEFRONT, graph=False, sync=True)
         kt = ctx.kernel_times()
@@ -277,6 +284,15 @@ def run_gpu(args, rank, world, local):
             ctx.film_read_into(sid, fs[:3 * npix], fs[3 * npix:6 * npix], fs[6 * npix:])
             e2e_t.append(time.perf_counter() - t0)
         e2e_value = float(npix) * spp * world / statistics.mean(e2e_t)
+
+        # counting replay of the timed passes (same seeds, counters on)
+        extend_kernel, counted = timed_variant(tuning, kt)
+        ctx.set_tuning_dict(counted)
+        ctx.set_counting(True)
+        ctx.render([sid], first, 1, seed=2024, mode=cg.CGPU_MODE_WAVEFRONT, graph=False, sync=True)
+        st = ctx.stats()
+        ctx.set_counting(False)
+        ctx.set_tuning_dict(tuning)
 
     # roofline of the dominant kernel (closest-hit traversal), algorithmic bytes:
     # 64 B per quantized 4-wide node + 48 B per triangle record + 64 B ray/hit queue I/O
@@ -328,7 +344,7 @@ def run_gpu(args, rank, world, local):
                  "tie_rule_fraction_of_closest": st.tie_rays / max(1, st.closest_rays)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                     "kernel": "k_wf_extend_pww (closest-hit traversal)",
+                     "kernel": extend_kernel + " (closest-hit traversal)",
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6.8 TB/s",
                      "limiter": "not HBM: the BVH and triangles sit in the 129 MB L2; issue slots and "
                                 "L1/L2 latency under divergence (lanes per warp instruction below)",

@@ -450,8 +450,9 @@ cgpu_status cgpu_set_adjoint_mode(cgpu_ctx* ctx, int32_t mode);
 
 /* Per-kernel CUDA-event timing of the following renders (launches are made
  * one by one instead of through the captured graph while it is on, and the
- * shadow pass runs after the extend pass instead of beside it, so that each
- * kernel is timed alone). */
+ * ray passes of a bounce run one after the other, each a launch of its own,
+ * instead of side by side or, with one ray per thread, in one launch; so that
+ * each kernel is timed alone). */
 enum {
     CGPU_KERNEL_GENERATE = 0,
     CGPU_KERNEL_EXTEND = 1,     /* closest-hit traversal of continuation rays */
