@@ -96,7 +96,7 @@ inline size_t wf_layout(char* base, size_t cap, int cnt_rows, WfBuffers* w) {
         w->q_mocc[k] = reinterpret_cast<int*>(take(cap * sizeof(int)));
     }
     for (int k = 0; k < kNumBsdfKinds; ++k) w->q_mat[k] = reinterpret_cast<int*>(take(cap * sizeof(int)));
-    w->q_tie = reinterpret_cast<int*>(take(2 * cap * sizeof(int)));
+    w->q_tie = reinterpret_cast<int*>(take(cap * sizeof(int)));
     w->cnt = reinterpret_cast<int*>(take(size_t(cnt_rows) * kCntStride * sizeof(int)));
     w->cnt_depth = cnt_rows;
     return off;

@@ -964,11 +964,11 @@ uint32_t scan_launches(uint32_t n) {
     return 1 + (nb > 1 ? scan_launches(nb) + 1 : 0);
 }
 
-// Ray reordering buffers for 2 * path_cap queue entries (continuation + MIS
-// rays of a pass), kept while tuning.reorder is on.
+// Ray reordering buffers for the path_cap rays a closest-hit pass can have, kept
+// while tuning.reorder is on.
 cgpu_status ensure_sort_buffers(cgpu_ctx* ctx) {
     if (!ctx->tuning.reorder) return CGPU_OK;
-    const uint64_t cap = uint64_t(ctx->path_cap) * 2;
+    const uint64_t cap = ctx->path_cap;
     if (ctx->sort_block && ctx->sort_cap >= cap) return CGPU_OK;
     if (ctx->sort_block) cudaFree(ctx->sort_block);
     ctx->sort_block = nullptr;
@@ -1110,7 +1110,7 @@ cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool cou
     const int sort_bits = ctx->tuning.reorder == 1 ? 9 : ctx->tuning.reorder == 2 ? 7 : ctx->tuning.reorder == 3 ? 4 : 0;
     const int sort_passes = (3 + 3 * sort_bits + 7) / 8;
     if (reorder) a.sorted = ctx->sort.vals[sort_passes & 1];
-    const int gkeys = grid_for(ctx, k_ray_keys, 256, uint64_t(paths) * 2);
+    const int gkeys = grid_for(ctx, k_ray_keys, 256, paths);
     // the persistent passes keep the bottom of their traversal stacks in shared memory
     const size_t ext_sm = stack_smem(ext_kernel, trav >= 2, true, bt);
     const size_t ext_sorted_sm = stack_smem(ext_sorted, trav >= 2, true, bt);
