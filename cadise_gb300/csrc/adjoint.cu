@@ -324,6 +324,7 @@ cgpu_status cgpu_adjoint_backward(cgpu_ctx* ctx, int32_t scene, uint32_t spp, ui
         if (ws != CGPU_OK) {
             cudaStreamSynchronize(ctx->stream);
             release_grad(g);
+            cg_adjoint_trim(ctx);
             return ws;
         }
     } else if (e == cudaSuccess) {
@@ -361,6 +362,7 @@ cgpu_status cgpu_adjoint_backward(cgpu_ctx* ctx, int32_t scene, uint32_t spp, ui
         e = cudaMemcpyAsync(grad_radiance, g.gl, size_t(3 * nlight) * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
     const cgpu_status fin = e != cudaSuccess ? cg_cuda(ctx, e, "adjoint_backward") : cg_check_status(ctx, "adjoint_backward");
     release_grad(g);
+    cg_adjoint_trim(ctx);
     return fin;
 }
 

@@ -302,7 +302,7 @@ struct cgpu_ctx {
     uint32_t path_cap = 0;
     cg::WfBuffers wf{};
     void* wf_block = nullptr;
-    // wavefront adjoint state (Ltot, acc, records), kept between calls
+    // wavefront adjoint state (Ltot, acc, records), kept between calls up to a size (cg_adjoint_trim)
     // ray reordering buffers (allocated while tuning.reorder is on)
     uint32_t sort_cap = 0;
     cg::SortBufs sort{};
@@ -362,6 +362,8 @@ cgpu_status cg_camera(cgpu_ctx* ctx, int scene, const double* d_xy, uint32_t n, 
 cgpu_status cg_film_clear(cgpu_ctx* ctx, int scene);
 void cg_free_render_state(cgpu_ctx* ctx);
 void cg_drop_graphs(cgpu_ctx* ctx);
+// After a backward call: gives a large adjoint state back.
+void cg_adjoint_trim(cgpu_ctx* ctx);
 
 // implemented in api.cu
 cgpu_status cg_fail(cgpu_ctx* ctx, cgpu_status s, const std::string& msg);

@@ -1511,6 +1511,10 @@ namespace {
 // Most bytes of records a batch takes: 13 million paths of depth 12 through three
 // kinds of material.  Beyond that the frame is done in parts.
 constexpr uint64_t kAdjRecordBytes = uint64_t(4) << 30;
+// Most bytes of state and records the context keeps between calls (all of a batch
+// of 11 million paths of depth 6 through two kinds of material); what is larger is
+// given back when the call ends.
+constexpr size_t kAdjKeep = size_t(2) << 30;
 
 // The launches of bounce b of a batch with records: hits and shade queues are
 // the row's own, and so are the outcomes of the rays that the shadow and MIS
@@ -1544,7 +1548,7 @@ void enqueue_adjoint_replay(cgpu_ctx* ctx, RenderArgs a, const AdjRecords& rec, 
     }
 }
 
-// Room for the adjoint state of *paths paths, kept between calls.  Where the
+// Room for the adjoint state of *paths paths (cg_adjoint_trim).  Where the
 // device has not that much left, *paths is halved until it has.
 cgpu_status ensure_adj_buffers(cgpu_ctx* ctx, int depth, uint32_t* paths, AdjBufs* a, AdjRecords* r) {
     cudaError_t e = cudaSuccess;
@@ -1571,6 +1575,13 @@ cgpu_status ensure_adj_buffers(cgpu_ctx* ctx, int depth, uint32_t* paths, AdjBuf
 }
 
 }  // namespace
+
+void cg_adjoint_trim(cgpu_ctx* ctx) {
+    if (ctx->adj_bytes <= kAdjKeep) return;
+    cudaFree(ctx->adj_block);
+    ctx->adj_block = nullptr;
+    ctx->adj_bytes = 0;
+}
 
 cgpu_status cg_adjoint_wavefront(cgpu_ctx* ctx, int scene, uint32_t spp, uint64_t seed, const AdjBufs& params) {
     const SceneSlot& sl = ctx->scenes[scene];

@@ -6,6 +6,7 @@ import subprocess
 
 import pytest
 
+import cadise_gb300 as cg
 from cadise_gb300 import scenes
 
 ROOT = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
@@ -28,6 +29,24 @@ def test_wavefront_state(ly):
     counters a bounce, in a block of whole 256 bytes."""
     paths = 1 << 20
     assert ly.ly_wavefront_bytes(paths, 34) <= paths * (14 * 16 + 14 * 4) + 34 * 64 + 255
+
+
+@pytest.mark.gpu
+def test_adjoint_records_kept_by_a_context():
+    """The records of a deep frame (4 GiB a batch) are given back when the call ends:
+    a context keeps 2 GiB at most, and the calls that follow give the same."""
+    import numpy as np
+    import torch
+    with cg.Context(device=0) as ctx:
+        sid = ctx.upload(scenes.diff_scene(width=1024, height=1024, spp=4, max_depth=200, n_spheres=6, subdivision=1,
+                                           tex_size=8, n_conductors=2, n_lights=2, seed=5))
+        W = np.full((1024, 1024, 3), 1e-3, np.float32)
+        ctx.adjoint_forward(sid, 1, 3)  # the path state and the gradient buffers
+        before = torch.cuda.mem_get_info()[0]
+        first = ctx.adjoint_backward(sid, 1, 3, W)
+        assert before - torch.cuda.mem_get_info()[0] < (2 << 30) + (64 << 20)
+        for a, b in zip(first, ctx.adjoint_backward(sid, 1, 3, W)):
+            np.testing.assert_allclose(a, b, rtol=1e-9, atol=1e-12 * np.abs(a).max())
 
 
 @pytest.mark.gpu
