@@ -63,12 +63,12 @@ struct WfBuffers {
     float4* mis_h;
     uint4* meta;      // scene, pixel, sample, rng counter
     int* q_cont[2];
-    int* q_mis[2];
+    int* q_mis[2];    // laid out, not used: a MIS ray that meets its light goes to q_mocc
     int* q_shadow[2];
     int* q_mocc[2];   // MIS occlusion queries, ping-pong on the bounce
     int* q_mat[kNumBsdfKinds];
     // closest-hit rays whose persistent traversal met two primitives within
-    // the tie window (k_wf_extend_pww), for k_wf_ties: paths
+    // the tie reach (persistent_pass), for k_wf_ties: paths
     int* q_tie;
     int* cnt;
     int cnt_depth;    // bounces the counter array covers

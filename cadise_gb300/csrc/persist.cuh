@@ -17,7 +17,7 @@
 //  * A node comes in two 32-byte loads instead of four of 16 (L1 tag look-ups
 //    halved).
 // Closest-hit passes of the 1 M-triangle 1080p frame, 16 samples a pixel:
-// 52.5 -> 34.4 ms; any-hit passes 25.0 -> 17.6 ms.
+// 52.5 ms with the inner loops, 34.1 here; any-hit passes 25.0 and 17.8 ms.
 #pragma once
 
 #include "traverse.cuh"
@@ -43,8 +43,8 @@ constexpr int kRoundSteps = 6;
 // (2 in 100,000 on the million-triangle field) moves its oldest kSpill entries
 // to local memory and takes them back when it has emptied the rest.
 // Closest hit: an entry is (child entry, distance); any hit: the child entry.
-// More rows cost L1 capacity, fewer cost spills: 16 rows 39.7 ms of closest-hit
-// passes, 12 rows 40.6, 11 rows 41.6 (an earlier form of the pass).
+// More rows cost L1 capacity, fewer cost spills: 16 rows 34.1 ms of closest-hit
+// passes, 12 rows 36.3, 11 rows 37.5.
 constexpr int kSmemStack = 16, kSpill = 8;
 // the dynamic shared memory of a persistent traversal launch
 extern __shared__ __align__(16) uint32_t trav_stack_smem[];

@@ -354,12 +354,13 @@ __global__ void k_wf_extend_dyn(RenderArgs a, int b) {
 }
 
 // Registers of the persistent passes: 18 blocks of 64 threads an SM.  The
-// 1 M-triangle frame's closest-hit passes take 33.9 ms at 56 registers (32 bytes
-// of spills in the ray set-up), 34.6 at 64 and 37.3 at 48.
+// 1 M-triangle frame's closest-hit / any-hit passes (16 samples) take 34.0 / 17.8
+// ms at 56 registers (36 bytes of spills in the ray set-up of the closest-hit
+// pass), 34.0 / 18.2 at 64 and 35.6 / 19.0 at 48.
 constexpr int kPersistRegs = 56;
 
 // Persistent closest-hit pass (persist.cuh) over the continuation rays.  A ray
-// that meets two primitives within the tie window is left to k_wf_ties.
+// that meets two primitives within the tie reach is left to k_wf_ties.
 template <bool COUNT, bool SPH, bool SORTED = false>
 __global__ void __maxnreg__(kPersistRegs) k_wf_extend_pww(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
@@ -397,14 +398,15 @@ __global__ void __maxnreg__(kPersistRegs) k_wf_extend_pww(RenderArgs a, int b) {
 constexpr int kTieBlock = 64;
 
 // Closest-hit rays the persistent pass left to this kernel (q_tie): two
-// primitives within the tie window of each other, which tie_prefers orders
-// by the reference's own test and tie order (tie_hit).  Of two the pass has both
-// records and only the comparison is left; of more the ray is traced again with
-// the per-ray traversal.  Then it is finished as the persistent pass finishes its
-// other rays.  Bound by latency: few rays, and a launch that traces some of them
-// from their origins lasts about 100 us whatever their number.  It runs beside
-// the any-hit pass (on the other stream), and its grid strides over however few
-// rays it got.
+// primitives within the tie reach of the hit, of which tie_prefers orders those
+// within its window by the reference's own test and tie order (tie_hit).  Of two
+// the pass has both records and only the comparison is left; of more the ray is
+// traced again with the per-ray traversal.  Then it is finished as the persistent
+// pass finishes its other rays.  Bound by latency: few rays, and a launch that
+// traces some of them from their origins lasts about 100 us whatever their number
+// (2 M triangles under a sky, 33 launches: 3.5 ms; 1 M triangles, 26: 0.95).  It
+// runs beside the any-hit pass (on the other stream), and its grid strides over
+// however few rays it got.
 template <bool COUNT, bool SPH>
 __global__ void k_wf_ties(RenderArgs a, int b) {
     const WfBuffers& w = a.wf;
@@ -832,7 +834,7 @@ __global__ void k_trace(const SceneD* scenes, int scene, const cgpu_ray* rays, u
 // Large batches of queries: the persistent pass, then (closest hit) one thread
 // per ray for the answer.  k_query leaves the traversal's distance in hits[i].t,
 // its record slot in hits[i].primitive (-1: a miss) and the record within its
-// tie window in hits[i].u, as the pass reports it; k_query_resolve compares the
+// tie reach in hits[i].u, as the pass reports it; k_query_resolve compares the
 // two (tie_hit).
 CG_D void load_query(const cgpu_ray& r, float3* o, float3* d, float* tmin, float* tmax) {
     *o = mk(r.org[0], r.org[1], r.org[2]);
@@ -1148,7 +1150,7 @@ cgpu_status enqueue_wavefront(cgpu_ctx* ctx, int depth, uint32_t paths, bool cou
             timed(ctx, CGPU_KERNEL_EXTEND, s, [&] { ext_kernel<<<gext, bt, ext_sm, s>>>(a, b); });
         }
         if (trav >= 2) {
-            // the persistent pass's rays within the tie window
+            // the persistent pass's rays within the tie reach
             timed(ctx, CGPU_KERNEL_TIES, s, [&] { ties_kernel<<<gties, kTieBlock, 0, s>>>(a, b); });
             launches += 1;
         }
@@ -1652,8 +1654,8 @@ cgpu_status cg_adjoint_wavefront(cgpu_ctx* ctx, int scene, uint32_t spp, uint64_
 // buffer the call needs in a static array of this library, so that the call
 // itself allocates nothing.  Same kernels as cgpu_render; the batch tables are
 // written by a one-block setup kernel (arguments by value, no copies), and the
-// ray passes of a bounce are one launch on the context stream (with traversal 0;
-// else one after the other: no side stream, no events, no graph).
+// ray passes of a bounce are one launch on the context stream (with traversal 0
+// and 4; else one after the other: no side stream, no events, no graph).
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 

@@ -34,7 +34,7 @@ static_assert(sizeof(Bvh4Node) == 64, "Bvh4Node is 64 bytes");
 // float spacings of its coordinates), the origin at the union's lower plane,
 // every lower plane rounded down and every upper plane rounded up to a step.
 // The slab test computes (origin - o) / d + q * 2^e / d; its rounding error
-// is a few ulps of t, inside the traversal's 1 + 2 gamma(3) slack.  FP64
+// is a few ulps of t, inside the box tests' slack (box_widen).  FP64
 // arithmetic, so host and device encode alike.
 CG_HD void quantize_node(const float (&lo)[4][3], const float (&hi)[4][3], const uint32_t (&child)[4], int nk,
                          Bvh4Node* out) {
